@@ -48,6 +48,45 @@ int is_pow2_host(double x) {
     return (m == 0.5 || m == -0.5) ? 1 : 0;
 }
 
+/* Division by a run constant d in two operations (Brisebarre, Muller and
+ * Raina, IEEE Trans. Computers 53(8), 2004): with zh = 1/d rounded and zl =
+ * 1/d - zh rounded, fma(x, zh, x zl) misses x/d by less than 2^-50 of a unit
+ * in the last place before its rounding, so it is x/d correctly rounded
+ * unless x/d lies that close to the midpoint of two doubles. Those x, if any,
+ * are found here and tried: for integers X, D of 53 bits X/D is N / (2 D)
+ * units from a midpoint, where 2^e X - N is an odd multiple of D (e = 53 for
+ * X >= D, else 54), and only |N| <= 16 comes that close. True for 98.7 % of
+ * random divisors (and for the reciprocals of powers of two).
+ * Holds for every x whose products stay normal (|x| from 2^-900 to 2^900 for
+ * the d accepted here); below, the quotient may be off by one unit in the
+ * last place of a number of 1e-270. */
+bool reciprocal_pair(double d, double &zl) {
+    zl = 0.0;
+    int ex;
+    const double m = std::frexp(d, &ex);
+    if (!(m >= 0.5) || ex < -100 || ex > 100) return false;
+    const uint64_t D = (uint64_t)std::ldexp(m, 53);
+    const double dd = (double)D, hi = 1.0 / dd, lo = std::fma(-hi, dd, 1.0) / dd;
+    zl = std::ldexp(lo, 53 - ex);
+    const int t = __builtin_ctzll(D);
+    const uint64_t odd = D >> t;
+    if (t > 4) return true;   /* N is a multiple of 2^t */
+    auto mul = [&](uint64_t a, uint64_t b) { return (uint64_t)((unsigned __int128)a * b % odd); };
+    for (int e = 53; e <= 54; ++e) {
+        uint64_t inv = 1;   /* 2^-e mod odd */
+        for (int i = 0; i < e; ++i) inv = mul(inv, (odd + 1) / 2);
+        const uint64_t from = e == 53 ? D : uint64_t(1) << 52, to = e == 53 ? uint64_t(1) << 53 : D;
+        for (int N = -16; N <= 16; ++N) {
+            if (N == 0 || N % (1 << t) != 0) continue;
+            uint64_t X = mul(N > 0 ? (uint64_t)N : odd - (uint64_t)-N, inv);
+            if (X < from) X += (from - X + odd - 1) / odd * odd;
+            for (; X < to; X += odd)
+                if (std::fma((double)X, hi, (double)X * lo) != (double)X / dd) return false;
+        }
+    }
+    return true;
+}
+
 }  // namespace
 
 namespace cb {
@@ -117,6 +156,7 @@ StepConst make_const(const cb_params *p) {
     k.dx2 = k.dx * k.dx;
     k.inv_dx2 = 1.0 / k.dx2;
     k.dx2_pow2 = is_pow2_host(k.dx2);
+    k.dx2_pair = reciprocal_pair(k.dx2, k.inv_dx2_lo);
     k.dtf = (float)k.dt;
     k.dxf = (float)k.dx;
     k.dx2f = (float)k.dx2;
@@ -475,7 +515,7 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
     int tj, ns, parts;
     size_t sm;
     unsigned g;
-    if (h->k.temporal == 0 && nsteps > 2) h->k.temporal = choose_temporal(h);
+    if (h->p.d == 3 && h->k.temporal == 0 && nsteps > 2) h->k.temporal = choose_temporal(h);
     const int tl = h->k.temporal;
     const bool tb_ok = !h->expanding && h->unit_scale && tl > 1 &&
                        step3tb_geometry(h->k, h->prec, tl, tj, ns, sm, g, parts);
@@ -517,6 +557,25 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
             h->steps_done += tl;
             h->launches++;
             it += tl;
+            continue;
+        }
+        /* static 1-D and 2-D: several steps per launch, the last with its sums */
+        const bool fuse_sums = (flags & (CB_STEP_SUMS | CB_STEP_LOCAL)) == CB_STEP_SUMS;
+        const int fused = h->p.d <= 2 && h->unit_scale
+                              ? step2tb_steps(h->k, h->prec, plain_left + (fuse_sums ? 1 : 0), fuse_sums)
+                              : 0;
+        if (fused > 0) {
+            const bool sums_now = fuse_sums && it + fused - 1 == nsteps;
+            const int i = h->cphi, j = h->cpi;
+            e = launch_step2_tb(h->prec, h->k, fused, sums_now, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j],
+                                h->st, h->partials, h->stream);
+            if (e != cudaSuccess) return cuda_fail(h, e, "launching the temporally blocked step kernel");
+            h->cphi = 1 - i;
+            h->cpi = 1 - j;
+            for (int q = 0; q < fused; ++q) h->t += h->p.dt;   /* bubble.cpp:871, one addition per step */
+            h->steps_done += fused;
+            h->launches++;
+            it += fused;
             continue;
         }
         if (plain_left >= GRAPH_STEPS && graphs_wanted(h)) {

@@ -76,7 +76,9 @@ struct StepConst {
     float c2f, c3f, c4f, v2f, v3f, v4f, dvf;
     float dtf, dxf, dx2f, inv_dx2f;
     double dx, dx2, inv_dx2;
+    double inv_dx2_lo;  /* 1/dx2 - inv_dx2, rounded */
     int dx2_pow2;
+    int dx2_pair;       /* fma(x, inv_dx2, x inv_dx2_lo) is x / dx2 rounded (reciprocal_pair, cb_api.cpp) */
     double dxLD, mpl;
     int alpha, expanding;
     int want_local;
@@ -129,6 +131,13 @@ size_t step2_blocks(const StepConst &k);
 cudaError_t launch_step2(int prec, const StepConst &k, int sums, const void *phi_in, const void *pi_in,
                          void *phi_out, void *pi_out, void *le, void *lg, void *lp, DevState *st, double *partials,
                          cudaStream_t s);
+
+/* Several steps per launch on static 1-D and 2-D lattices (cb_step2_tb.cu).
+ * step2tb_steps: how many of the next `left` steps one launch takes, the last
+ * of the `left` measuring sums or not (0: the one-step kernels). */
+int step2tb_steps(const StepConst &k, int prec, int left, bool sums);
+cudaError_t launch_step2_tb(int prec, const StepConst &k, int steps, bool sums, const void *phi_in, const void *pi_in,
+                            void *phi_out, void *pi_out, DevState *st, double *partials, cudaStream_t s);
 
 /* d = 3 kernel with TMA-staged row tiles (cb_step3.cu). */
 bool step3_geometry(const StepConst &k, int prec, int &tj, int &nstage, size_t &smem, unsigned &grid);

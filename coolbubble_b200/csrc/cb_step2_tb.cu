@@ -1,0 +1,510 @@
+/* cb_step2_tb.cu -- several leapfrog steps per launch on static 1-D and 2-D
+ * lattices (Bubble::oneStep, src/bubble.cpp:849-876, for D = 1, 2; these
+ * backgrounds never expand, bubble.hpp:77, so between two reported lines no
+ * step needs a global sum).
+ *
+ * Overlapped tiling in registers. A block takes a tile of the lattice with a
+ * halo as deep as the number of steps, every thread holds a patch of it -- K
+ * rows of one 16-byte vector, phi and pi -- and the block advances the whole
+ * tile step by step; only the sites that no tile edge has reached yet are
+ * written back. Fields cross memory once per launch instead of once per step.
+ *
+ *  - d = 2: a warp holds K full rows of a tile (32 vectors wide), the block's
+ *    warps lie one below the other. Neighbours along axis 1 come from the
+ *    adjacent lanes by shuffle, along axis 0 from the thread's own registers;
+ *    only a patch's first and last rows go through shared memory, in two
+ *    buffers used in turn, so a step has one barrier.
+ *  - d = 1: a warp holds K vectors of a row of 32 K vectors; a step has no
+ *    barrier and no shared memory.
+ *  - Coordinates wrap, so tiles that hang over the lattice's end and lattices
+ *    smaller than a tile need no special case. n that is no multiple of the
+ *    vector width loads and stores site by site (once per launch).
+ *  - The last step of a launch may measure the box averages (bubble.cpp:
+ *    761-844), in double per thread and across threads, in a fixed order.
+ *
+ * What bounds it: the arithmetic of the tile, halo included. ncu, 8 steps on
+ * 4096^2 floats: FMA pipe 62 % busy (the packed operations occupy it two
+ * cycles), DRAM 21 %; 4 steps on 3072^2 doubles: FP64 pipe 60-65 %, DRAM 32 %.
+ * us per step, one launch per step -> here: 512^2 double 2.72 -> 1.10, 1000^2
+ * float 6.69 -> 1.34, 3072^2 double (dx^2 no power of two) 52.2 -> 24.9,
+ * 4096^2 float 47.3 -> 14.4; 4096 sites (d = 1, double) 2.19 -> 0.16.
+ *
+ * The per-site operations are those of the one-step kernels (cb_step.cu,
+ * cb_step2.cu) for a = 1, where a^(d-2) = a^d = 1 and the products with them
+ * are exact: fields are identical to theirs bit for bit.
+ */
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "cb_internal.h"
+#include "cb_launch.cuh"
+#include "cb_step_common.cuh"
+#include "cb_tma.cuh"
+
+namespace cb {
+
+int sm_count();
+
+namespace {
+
+constexpr int TB2_MAXW = 16;    /* warps per block at most */
+
+/* How the Laplacian is divided by dx^2, always correctly rounded: by its
+ * reciprocal (float, or dx^2 a power of two: exact), by the reciprocal as a
+ * pair of doubles (dx2_pair; 3072^2: 23.0 us per step against 22.9 with the
+ * one product, and 31.5 with a quotient refined twice), or, where neither
+ * holds, by the compiler's division. */
+enum { BY_MUL = 0, BY_PAIR = 1, BY_DIV = 2 };
+
+/* constants of the update (a = 1) */
+template <typename T>
+struct Cst;
+template <>
+struct Cst<float> {
+    F2 idx2, dt, nc2, c3, nc4;
+    __device__ __forceinline__ explicit Cst(const StepConst &k)
+        : idx2(f2_splat(k.inv_dx2f)), dt(f2_splat(k.dtf)), nc2(f2_splat(-k.c2f)), c3(f2_splat(k.c3f)),
+          nc4(f2_splat(-k.c4f)) {}
+};
+template <>
+struct Cst<double> {
+    const StepConst &k;
+    __device__ __forceinline__ explicit Cst(const StepConst &kk) : k(kk) {}
+};
+
+/* One packed pair: the force with the periodic Laplacian and V'(phi) (the
+ * exact negation of the one-step kernel's rounded V'/phi), kick and drift. */
+template <int D>
+__device__ __forceinline__ void pair2(const Cst<float> &K, F2 cc, F2 um, F2 up, F2 km, F2 kp, F2 &pi, F2 &phi) {
+    const F2 two = f2_add(cc, cc);
+    F2 lap = f2_add(f2_sub(kp, two), km);
+    if (D == 2) lap = f2_add(f2_add(f2_sub(up, two), um), lap);
+    const F2 nh = f2_fma(cc, f2_fma(cc, K.nc4, K.c3), K.nc2);
+    const F2 force = f2_fma(lap, K.idx2, f2_mul(cc, nh));
+    pi = f2_fma(K.dt, force, pi);
+    phi = f2_fma(K.dt, pi, cc);
+}
+
+/* One vector of one step: c its sites, um / up the vectors one row before and
+ * after along axis 0 (d = 2), l / r the sites beside it; pi advances in place. */
+template <int D, int BY>
+__device__ __forceinline__ float4 update(const Cst<float> &K, const float4 &c, const float4 &um, const float4 &up,
+                                         float l, float r, float4 &p) {
+    const F2 mid = f2_pack(c.y, c.z);
+    F2 pa = f2_pack(p.x, p.y), pb = f2_pack(p.z, p.w), fa, fb;
+    pair2<D>(K, f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(l, c.x), mid, pa, fa);
+    pair2<D>(K, f2_pack(c.z, c.w), f2_pack(um.z, um.w), f2_pack(up.z, up.w), mid, f2_pack(c.w, r), pb, fb);
+    p = make_float4(f2_lo(pa), f2_hi(pa), f2_lo(pb), f2_hi(pb));
+    return make_float4(f2_lo(fa), f2_hi(fa), f2_lo(fb), f2_hi(fb));
+}
+template <int BY>
+__device__ __forceinline__ double over_dx2(const StepConst &k, double lap) {
+    if (BY == BY_PAIR) return __fma_rn(lap, k.inv_dx2, __dmul_rn(lap, k.inv_dx2_lo));
+    return BY == BY_MUL ? __dmul_rn(lap, k.inv_dx2) : __ddiv_rn(lap, k.dx2);
+}
+template <int D, int BY>
+__device__ __forceinline__ double site(const StepConst &k, double c, double um, double up, double l, double r,
+                                       double &p) {
+    using A = Ar<double>;
+    const double two = A::add(c, c);
+    const double tk = A::add(A::sub(r, two), l);
+    const double lap = D == 2 ? A::add(A::add(A::sub(up, two), um), tk) : tk;
+    p = A::add(p, A::mul(k.dt, A::sub(over_dx2<BY>(k, lap), dV<double>(k, c))));
+    return A::add(c, A::mul(k.dt, p));
+}
+template <int D, int BY>
+__device__ __forceinline__ double2 update(const Cst<double> &K, const double2 &c, const double2 &um,
+                                          const double2 &up, double l, double r, double2 &p) {
+    double2 f;
+    f.x = site<D, BY>(K.k, c.x, um.x, up.x, l, c.y, p.x);
+    f.y = site<D, BY>(K.k, c.y, um.y, up.y, c.x, r, p.y);
+    return f;
+}
+
+/* The box sums of one vector (the one-step kernels' expressions); pn: pi after
+ * the kick, po: before it. */
+template <typename T, int D>
+struct Measure {
+    using A = Ar<T>;
+    using V = typename Vec<T>::V;
+    T kin_w, vel_w, adx, inv_adx;
+    bool mul;   /* multiply by 1 / (a dx): float, or exact */
+    __device__ __forceinline__ T grad(T x) const { return mul ? A::mul(x, inv_adx) : A::div(x, adx); }
+    __device__ __forceinline__ void add(const StepConst &k, const V &c, const V &dn, T right, const V &pn, const V &po,
+                                        bool whole, int valid, double (&acc)[NSUM]) const {
+        constexpr int W = Vec<T>::W;
+#pragma unroll
+        for (int s = 0; s < W; ++s) {
+            if (!whole && s >= valid) break;
+            const T cur = Vec<T>::get(c, s);
+            const T gx = grad(A::sub(s == W - 1 ? right : Vec<T>::get(c, s < W - 1 ? s + 1 : s), cur));
+            const T gy = D == 2 ? grad(A::sub(Vec<T>::get(dn, s), cur)) : (T)0;
+            const T gz = (T)0;
+            const T eg = A::mul((T)0.5, A::add(A::add(A::sq(gx), A::sq(gy)), A::sq(gz)));
+            const T ep = Vpot<T>(k, cur);
+            const T pin = Vec<T>::get(pn, s), pio = Vec<T>::get(po, s);
+            const T ek = A::mul(A::mul(kin_w, pin), pin);
+            const T v = A::mul(pin, vel_w);
+            const T et = A::add(A::add(ek, eg), ep);
+            auto put = [&](int i, T x) { acc[i] = __dadd_rn(acc[i], (double)x); };
+            put(S_EK, ek);
+            put(S_EP, ep);
+            put(S_EG, eg);
+            put(S_PHI, cur);
+            put(S_V, v);
+            put(Q_EK, A::sq(ek));
+            put(Q_EP, A::sq(ep));
+            put(Q_EG, A::sq(eg));
+            put(Q_ET, A::sq(et));
+            put(Q_PHI, A::sq(cur));
+            put(Q_V, A::sq(v));
+            put(S_EKIN_IN, A::mul(A::mul(kin_w, pio), pio));
+        }
+    }
+};
+
+template <int B>
+__device__ __forceinline__ void cp_async(uint32_t to, const void *from) {
+    if constexpr (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(from) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(B) : "memory");
+}
+
+/* tx x ty: the sites a tile writes (columns x rows), hx its column halo (a
+ * multiple of the vector width, at least `steps`), tiles_x x tiles_y tiles. */
+struct Tiles {
+    int tx, ty, hx, tiles_x, tiles;
+};
+
+template <typename T, int D, int K, bool ALIGNED, int BY, bool SUMS>
+__global__ void __launch_bounds__(TB2_MAXW * 32, 1)
+    k_step2_tb(StepConst k, Tiles g, int steps, const T *__restrict__ phi_in, const T *__restrict__ pi_in,
+               T *__restrict__ phi_out, T *__restrict__ pi_out, DevState *st, double *partials) {
+    using VV = Vec<T>;
+    using V = typename VV::V;
+    constexpr int W = VV::W;
+    /* first and last rows of every warp's patch, two buffers */
+    extern __shared__ __align__(16) unsigned char smraw[];
+    V *const edge = reinterpret_cast<V *>(smraw);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int n = k.n;
+    const Cst<T> C(k);
+    double acc[NSUM];
+    Measure<T, D> M{};
+    pdl_wait();   /* the previous launch's fields and device state */
+    if (SUMS) {
+#pragma unroll
+        for (int s = 0; s < NSUM; ++s) acc[s] = 0.0;
+        M.kin_w = (T)st->kin_w;
+        M.vel_w = (T)st->vel_w;
+        M.adx = (T)st->adx;
+        M.inv_adx = (T)st->inv_adx;
+        M.mul = std::is_same<T, float>::value || st->adx_pow2 != 0;
+    }
+    /* where a tile starts, and this thread's column of vector r and row of it,
+     * counted from the first site the tile (d = 1: the warp's part of it) writes */
+    auto x_of = [&](int tile) { return (D == 1 ? tile * nw + w : tile % g.tiles_x) * g.tx; };
+    auto y_of = [&](int tile) { return D == 1 ? 0 : tile / g.tiles_x * g.ty; };
+    auto col = [&](int r) { return (lane + (D == 1 ? 32 * r : 0)) * W - g.hx; };
+    auto row = [&](int r) { return D == 1 ? 0 : w * K + r - steps; };
+    auto wrap = [&](int i) {
+        i %= n;
+        return i < 0 ? i + n : i;
+    };
+    /* each thread copies its own patch of the next tile into its own shared
+     * slots while the block computes the current one: no barrier is involved */
+    V *const mine = edge + (D == 2 ? 2 * 64 * nw : 0) + threadIdx.x;
+    auto fetch = [&](int tile) {
+        const int x0 = x_of(tile);
+        int c = wrap(x0 + col(0)), y = wrap(y_of(tile) + row(0));
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            const size_t base = (size_t)y * n;
+            const uint32_t to = smem_u32(mine + 2 * r * blockDim.x), step_b = 16u * blockDim.x;
+            if (ALIGNED) {
+                cp_async<16>(to, phi_in + base + c);
+                cp_async<16>(to + step_b, pi_in + base + c);
+            } else {
+                int cs = c;
+#pragma unroll
+                for (int s = 0; s < W; ++s) {
+                    cp_async<sizeof(T)>(to + s * sizeof(T), phi_in + base + cs);
+                    cp_async<sizeof(T)>(to + step_b + s * sizeof(T), pi_in + base + cs);
+                    if (++cs == n) cs = 0;
+                }
+            }
+            if (D == 1) c = wrap(x0 + col(r + 1));
+            else if (++y == n) y = 0;
+        }
+    };
+    if ((int)blockIdx.x < g.tiles) fetch(blockIdx.x);
+    int buf = 0;   /* the edge rows' buffer of the next step: in turn, over all the block's tiles */
+    for (int tile = blockIdx.x; tile < g.tiles; tile += gridDim.x) {
+        /* this thread's patch: column of vector r, and row of it, counted from
+         * the first site the tile (d = 1: the warp's part of it) writes */
+        const int x0 = x_of(tile), y0 = y_of(tile);
+        V phi[K], pi[K];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            phi[r] = mine[2 * r * blockDim.x];
+            pi[r] = mine[(2 * r + 1) * blockDim.x];
+        }
+        if (tile + gridDim.x < g.tiles) fetch(tile + gridDim.x);
+        /* sites of vector r that this tile writes: none, or the first `valid` */
+        auto valid_of = [&](int r) -> int {
+            const int c = col(r), y = row(r);
+            if (c < 0 || c >= g.tx || (D == 2 && (y < 0 || y >= g.ty || y0 + y >= n))) return 0;
+            return min(W, n - (x0 + c));
+        };
+        auto step = [&](auto measure) {
+            constexpr bool MEASURE = decltype(measure)::value;
+            V prev = phi[0], below = phi[K - 1];
+            if (D == 2) {
+                V *const e = edge + buf * (64 * nw);
+                buf ^= 1;
+                e[(2 * w) * 32 + lane] = phi[0];
+                e[(2 * w + 1) * 32 + lane] = phi[K - 1];
+                __syncthreads();
+                if (w > 0) prev = e[(2 * w - 1) * 32 + lane];
+                if (w + 1 < nw) below = e[(2 * w + 2) * 32 + lane];
+            }
+            T last = VV::get(phi[0], W - 1);   /* d = 1: the last site of the row's previous vector */
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const V cur = phi[r];
+                const V next = r < K - 1 ? phi[r < K - 1 ? r + 1 : r] : below;
+                T left = __shfl_up_sync(0xffffffffu, VV::get(cur, W - 1), 1);
+                T right = __shfl_down_sync(0xffffffffu, VV::get(cur, 0), 1);
+                if (D == 1) {
+                    const T before = __shfl_sync(0xffffffffu, last, 31);
+                    const T after = __shfl_sync(0xffffffffu, VV::get(next, 0), 0);
+                    if (lane == 0) left = before;
+                    if (lane == 31) right = after;
+                    last = VV::get(cur, W - 1);
+                }
+                const V before_kick = pi[r];
+                phi[r] = update<D, BY>(C, cur, prev, next, left, right, pi[r]);
+                if (MEASURE) {
+                    const int valid = valid_of(r);
+                    if (valid > 0) M.add(k, cur, next, right, pi[r], before_kick, ALIGNED, valid, acc);
+                }
+                prev = cur;
+            }
+        };
+        const int plain = SUMS ? steps - 1 : steps;
+        for (int s = 0; s < plain; ++s) step(std::false_type{});
+        if (SUMS) step(std::true_type{});
+#pragma unroll
+        for (int r = 0; r < K; ++r) {
+            const int valid = valid_of(r);
+            if (valid <= 0) continue;
+            const size_t o = (size_t)(y0 + row(r)) * n + x0 + col(r);
+            if (ALIGNED) {
+                *reinterpret_cast<V *>(phi_out + o) = phi[r];
+                *reinterpret_cast<V *>(pi_out + o) = pi[r];
+            } else {
+#pragma unroll
+                for (int s = 0; s < W; ++s)
+                    if (s < valid) {
+                        phi_out[o + s] = VV::get(phi[r], s);
+                        pi_out[o + s] = VV::get(pi[r], s);
+                    }
+            }
+        }
+    }
+    pdl_allow_next();
+
+    if (SUMS) {
+        /* the block's row of partial sums, then the last block's total: warps by
+         * shuffle, warps in order, blocks in the order of sum_rows */
+        __shared__ double red[TB2_MAXW][NSUM];
+        __shared__ double tot[NSUM];
+        __shared__ bool is_last;
+#pragma unroll
+        for (int s = 0; s < NSUM; ++s) {
+            double x = acc[s];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x = __dadd_rn(x, __shfl_down_sync(0xffffffffu, x, o));
+            if (lane == 0) red[w][s] = x;
+        }
+        __syncthreads();
+        if (threadIdx.x < NSUM) {
+            double x = 0.0;
+            for (int i = 0; i < nw; ++i) x = __dadd_rn(x, red[i][threadIdx.x]);
+            partials[(size_t)blockIdx.x * NSUM + threadIdx.x] = x;
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            is_last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
+            if (is_last) st->counter = 0u;
+        }
+        __syncthreads();
+        if (!is_last) return;
+        __threadfence();
+        /* warp w adds sums w, w + nw, ...: lane l the rows l, l + 32, ... */
+        for (int s = w; s < NSUM; s += nw) {
+            double x = 0.0;
+            for (unsigned b = lane; b < gridDim.x; b += 32) x = __dadd_rn(x, __ldcg(partials + (size_t)b * NSUM + s));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x = __dadd_rn(x, __shfl_down_sync(0xffffffffu, x, o));
+            if (lane == 0) tot[s] = x;
+        }
+        __syncthreads();
+        if (threadIdx.x < 32) epilogue(k, st, tot, true, true, lane);
+    }
+}
+
+}  // namespace
+
+namespace {
+
+/* How a launch of `steps` steps tiles the lattice. */
+struct Plan2 {
+    int rows = 0, warps = 0;   /* K of the patches, warps per block */
+    Tiles g{};
+    unsigned grid = 0;
+    double us = 0.0;           /* modelled time */
+};
+
+constexpr int TB2_STEPS = 20;   /* d = 2: steps per launch at most (the halo eats the tile beyond) */
+
+/* d = 2: the patch height and block size whose modelled time is least. A
+ * launch costs a start, then per round of resident blocks a load and a store
+ * of the rows the busiest SM holds, and per step a latency and an issue time
+ * per row (a row: 32 vectors; 8-row patches pay for 128 registers with fewer
+ * warps to hide latency). The coefficients, in us, were fitted to 418 timed
+ * (n, K, warps, steps) combinations of each precision, n from 64 to 3072:
+ * 7 % rms off, and the plan it picks within 6 % of the fastest one timed
+ * (9 % at 3072^2 in double). Small lattices so get small blocks on many SMs
+ * and few steps per launch, large ones tall tiles whose halo costs less. */
+bool plan_2d(const StepConst &k, int prec, int steps, Plan2 &best) {
+    struct Cost { double start, load, load_row, step, row4, row8, wide; };
+    static constexpr Cost cost[2] = {{1.60, -0.16, 0.030, 0.120, 0.0079, 0.0100, 0.061},    /* double */
+                                     {1.54, 0.11, 0.027, 0.066, 0.0049, 0.0069, 0.088}};    /* float */
+    static constexpr int shape[5][2] = {{4, 4}, {4, 8}, {4, 16}, {8, 8}, {8, 16}};
+    const Cost &c = cost[prec == P_FP64 ? 0 : 1];
+    const int W = prec == P_FP64 ? 2 : 4, sms = sm_count();
+    best.us = 0.0;
+    for (const auto &s : shape) {
+        Plan2 p;
+        p.rows = s[0];
+        p.warps = s[1];
+        p.g.hx = (steps + W - 1) / W * W;
+        p.g.tx = 32 * W - 2 * p.g.hx;
+        p.g.ty = p.rows * p.warps - 2 * steps;
+        if (p.g.tx <= 0 || p.g.ty <= 0) continue;
+        p.g.tiles_x = (k.n + p.g.tx - 1) / p.g.tx;
+        const long long tiles = (long long)p.g.tiles_x * ((k.n + p.g.ty - 1) / p.g.ty);
+        const int per_sm = TB2_MAXW / p.warps;
+        p.g.tiles = (int)tiles;
+        p.grid = (unsigned)std::min<long long>(tiles, (long long)sms * per_sm);
+        const long long busiest = (tiles + sms - 1) / sms;
+        auto round_us = [&](long long blocks) {
+            const double rows = (double)blocks * p.rows * p.warps;
+            return c.load + c.load_row * rows +
+                   steps * (c.step + (p.rows == 4 ? c.row4 : c.row8) * rows + (p.warps == TB2_MAXW ? c.wide : 0.0));
+        };
+        p.us = c.start + (double)(busiest / per_sm) * round_us(per_sm) +
+               (busiest % per_sm ? round_us(busiest % per_sm) : 0.0);
+        if (best.us == 0.0 || p.us < best.us) best = p;
+    }
+    return best.us > 0.0;
+}
+
+/* d = 1: warps are independent, so only the patch length matters: two vectors
+ * per thread below 2^18 sites (more warps: 4096 double sites 0.15 us per step,
+ * 0.17 with four), four from there on (2^20 floats 0.49 against 0.55 us). */
+constexpr int TB1_STEPS = 32;
+bool plan_1d(const StepConst &k, int prec, int steps, Plan2 &p) {
+    const int W = prec == P_FP64 ? 2 : 4;
+    p.rows = k.n < (1 << 18) ? 2 : 4;
+    p.warps = 4;
+    p.g.hx = (steps + W - 1) / W * W;
+    p.g.tx = 32 * W * p.rows - 2 * p.g.hx;
+    if (p.g.tx <= 0) return false;
+    p.g.ty = 1;
+    p.g.tiles_x = (k.n + p.g.tx - 1) / p.g.tx;
+    p.g.tiles = (p.g.tiles_x + p.warps - 1) / p.warps;
+    p.grid = (unsigned)std::min(p.g.tiles, sm_count() * (TB2_MAXW / p.warps));
+    return true;
+}
+
+bool plan2(const StepConst &k, int prec, int steps, Plan2 &p) {
+    return k.d == 1 ? plan_1d(k, prec, steps, p) : plan_2d(k, prec, steps, p);
+}
+
+}  // namespace
+
+/* The steps of the next launch when `left` steps are to come, the last of them
+ * with sums or not: launches of nearly equal depth, as many as the modelled
+ * time is least for. A single step without sums is left to the one-step
+ * kernels (512^2 double: 2.7 us, here 3.1). */
+int step2tb_steps(const StepConst &k, int prec, int left, bool sums) {
+    if (k.d > 2 || k.force_generic || k.temporal == 1 || left < 1 || (left == 1 && !sums)) return 0;
+    if (k.d == 1) {
+        /* in double a halo of 32 of 256 sites costs more than a launch from 2^18 sites on */
+        const int most = prec == P_FP64 && k.n >= (1 << 18) ? TB1_STEPS / 2 : TB1_STEPS;
+        const int launches = (left + most - 1) / most;
+        return (left + launches - 1) / launches;
+    }
+    int steps = 0;
+    double least = 0.0;
+    for (int t = std::min(left, TB2_STEPS); t >= 1; --t) {
+        const int launches = (left + t - 1) / t;
+        if ((left + launches - 1) / launches != t) continue;   /* not the even split of its launches */
+        Plan2 p;
+        if (!plan_2d(k, prec, t, p)) continue;
+        if (steps == 0 || launches * p.us < least) {
+            steps = t;
+            least = launches * p.us;
+        }
+    }
+    return steps;
+}
+
+cudaError_t launch_step2_tb(int prec, const StepConst &k, int steps, bool sums, const void *phi_in, const void *pi_in,
+                            void *phi_out, void *pi_out, DevState *st, double *partials, cudaStream_t s) {
+    Plan2 p;
+    if (steps < 1 || !plan2(k, prec, steps, p)) return cudaErrorInvalidValue;
+    /* a block with sums writes a row of partial sums: no more of them than a run's
+     * one-step launches have (blocks take several tiles then) */
+    if (sums) p.grid = (unsigned)std::min<size_t>(p.grid, step_blocks(k));
+    const int W = prec == P_FP64 ? 2 : 4;
+    const bool aligned = k.n % W == 0;
+    const size_t smem = ((k.d == 2 ? (size_t)2 * 64 * p.warps : 0) + (size_t)2 * p.rows * 32 * p.warps) * 16;
+    auto go = [&](auto t, auto d, auto rows, auto al, auto dv, auto su) -> cudaError_t {
+        using T = decltype(t);
+        auto fn = k_step2_tb<T, decltype(d)::value, decltype(rows)::value, decltype(al)::value, decltype(dv)::value,
+                             decltype(su)::value>;
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(fn, dim3(p.grid), dim3(p.warps * 32), smem, s, k, p.g, steps, (const T *)phi_in,
+                          (const T *)pi_in, (T *)phi_out, (T *)pi_out, st, partials);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    auto with_rows = [&](auto t, auto d, auto al, auto dv, auto su) {
+        constexpr int less = decltype(d)::value == 1 ? 2 : 8;   /* d = 1: 2 or 4, d = 2: 4 or 8 */
+        return p.rows == 4 ? go(t, d, std::integral_constant<int, 4>{}, al, dv, su)
+                           : go(t, d, std::integral_constant<int, less>{}, al, dv, su);
+    };
+    auto with_sums = [&](auto t, auto d, auto al, auto dv) {
+        return sums ? with_rows(t, d, al, dv, Yes{}) : with_rows(t, d, al, dv, No{});
+    };
+    auto with_al = [&](auto t, auto d, auto dv) {
+        return aligned ? with_sums(t, d, Yes{}, dv) : with_sums(t, d, No{}, dv);
+    };
+    auto with_t = [&](auto d) {
+        using std::integral_constant;
+        if (prec != P_FP64) return with_al(0.f, d, integral_constant<int, BY_MUL>{});
+        if (k.dx2_pow2) return with_al(0.0, d, integral_constant<int, BY_MUL>{});
+        return k.dx2_pair ? with_al(0.0, d, integral_constant<int, BY_PAIR>{})
+                          : with_al(0.0, d, integral_constant<int, BY_DIV>{});
+    };
+    return k.d == 1 ? with_t(std::integral_constant<int, 1>{}) : with_t(std::integral_constant<int, 2>{});
+}
+
+}  // namespace cb
