@@ -389,14 +389,14 @@ int ensure_tmp(cb_handle *h, size_t bytes) {
     return CB_OK;
 }
 
-/* The temporal-block autotuner: for a static float 3-D run whose lattice the
+/* The temporal-block autotuner: for a static 3-D run whose lattice the
  * two-step pass can take, time one-step and two-step passes on the run's own
  * stream (each reads the current fields and writes the spare buffers, so the
  * run's state does not change) and keep whichever moves a step faster; the
- * choice is cached per device and lattice size. Both passes give the same
+ * choice is cached per device, lattice size and precision. Both passes give the same
  * fields bit for bit, so the choice only changes the speed. */
 int choose_temporal(cb_handle *h) {
-    if (h->expanding || !h->unit_scale || h->prec != P_FP32 || h->p.d != 3) return 1;
+    if (h->expanding || !h->unit_scale || h->p.d != 3) return 1;
     int tj, ns, parts;
     size_t sm;
     unsigned g;
@@ -405,7 +405,7 @@ int choose_temporal(cb_handle *h) {
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 1; }
     static std::mutex mu;
     static std::map<std::pair<int, int>, int> cache;
-    const std::pair<int, int> key(dev, h->p.n_grids);
+    const std::pair<int, int> key(dev, 2 * h->p.n_grids + (h->prec == P_FP64 ? 1 : 0));
     {
         std::lock_guard<std::mutex> lock(mu);
         auto it = cache.find(key);

@@ -51,13 +51,6 @@ namespace {
 
 constexpr int TB2_MAXW = 16;    /* warps per block at most */
 
-/* How the Laplacian is divided by dx^2, always correctly rounded: by its
- * reciprocal (float, or dx^2 a power of two: exact), by the reciprocal as a
- * pair of doubles (dx2_pair; 3072^2: 23.0 us per step against 22.9 with the
- * one product, and 31.5 with a quotient refined twice), or, where neither
- * holds, by the compiler's division. */
-enum { BY_MUL = 0, BY_PAIR = 1, BY_DIV = 2 };
-
 /* constants of the update (a = 1) */
 template <typename T>
 struct Cst;
@@ -98,11 +91,6 @@ __device__ __forceinline__ float4 update(const Cst<float> &K, const float4 &c, c
     pair2<D>(K, f2_pack(c.z, c.w), f2_pack(um.z, um.w), f2_pack(up.z, up.w), mid, f2_pack(c.w, r), pb, fb);
     p = make_float4(f2_lo(pa), f2_hi(pa), f2_lo(pb), f2_hi(pb));
     return make_float4(f2_lo(fa), f2_hi(fa), f2_lo(fb), f2_hi(fb));
-}
-template <int BY>
-__device__ __forceinline__ double over_dx2(const StepConst &k, double lap) {
-    if (BY == BY_PAIR) return __fma_rn(lap, k.inv_dx2, __dmul_rn(lap, k.inv_dx2_lo));
-    return BY == BY_MUL ? __dmul_rn(lap, k.inv_dx2) : __ddiv_rn(lap, k.dx2);
 }
 template <int D, int BY>
 __device__ __forceinline__ double site(const StepConst &k, double c, double um, double up, double l, double r,

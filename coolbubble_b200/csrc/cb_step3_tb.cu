@@ -5,14 +5,16 @@
  * reported ones needs a global sum). One launch reads phi_n, pi_{n-1/2} and
  * writes phi_{n+2}, pi_{n+3/2}: half the DRAM bytes per step.
  *
- *  - Tiles of TJ full rows of axis 1 (axis-2 neighbours wrap in shared
- *    memory); work items (plane part, tile) taken from a device-wide queue,
+ *  - Float and double; n any multiple of the 16-byte vector with rows of a warp
+ *    or more. Tiles of TJ full rows of axis 1 (axis-2 neighbours wrap in shared
+ *    memory; the last tile may hang over the lattice's end and repeat its first
+ *    rows); work items (plane part, tile) taken from a device-wide queue,
  *    part-major with tiles fastest (the items in flight share their halo rows
  *    in L2), one block per SM.
  *  - Input planes arrive by TMA bulk copies into a 4- to 6-stage ring: phi
  *    rows [j0 - 2, j0 + TJ + 2), pi rows [j0 - 1, j0 + TJ + 1) (periodic).
- *  - Each consumer thread owns the same positions in every plane (four of the
- *    tile, one of the two halo rows for some) and marches them along axis 0:
+ *  - Each consumer thread owns the same positions in every plane (two vectors of
+ *    the tile, a share of the two halo rows) and marches them along axis 0:
  *    its own columns of input phi, of level-1 phi and of level-1 pi stay in
  *    registers, so shared memory holds only what other threads read -- the
  *    input planes and two level-1 planes (TJ + 2 rows each). That leaves room
@@ -24,17 +26,24 @@
  *  - An item computing planes [p0, p1) streams input planes p0 - 2 .. p1 + 1
  *    (overlapped tiling: neighbouring items recompute the halo, no block
  *    talks to another). The input ring runs on from one item to the next.
- *  - The per-site results are those of the single-step kernel's float path
- *    (packed f32x2, the same rounded operations), so two blocked steps give
- *    the fields of two single steps bit for bit.
+ *  - The per-site results are those of the single-step kernel (float: packed
+ *    f32x2, the same rounded operations), so two blocked steps give the fields
+ *    of two single steps bit for bit.
+ *  - What bounds it: the latency of a round (load, two dependent updates, a
+ *    barrier) over 16 warps, ncu on 256^3: float FMA pipe 62 % busy, issue 55 %;
+ *    double FP64 pipe 36 %, issue 50 %; DRAM 41-47 %. us per step, one step per
+ *    pass -> here: 192^3 float 19.0 -> 17.1, 256^3 50.0 -> 27.9, 512^3 336 ->
+ *    197, 256^3 double 89 -> 63, 192^3 double 44.7 -> 29.9.
  *  - Waits are bounded (clock64 limit, sleeping retries); a timed-out block
  *    records an error word; consumer warps leave together (a vote in the
  *    per-round barrier).
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
 #include "cb_internal.h"
 #include "cb_launch.cuh"
@@ -55,125 +64,175 @@ constexpr int TB_IQ = 8;
 __device__ __forceinline__ bool tb_any(bool x) { return __syncthreads_or(x ? 1 : 0) != 0; }
 
 /* shared-memory accesses by 32-bit shared address */
-__device__ __forceinline__ float4 lds4(uint32_t a) {
+template <typename V>
+__device__ __forceinline__ V lds(uint32_t a);
+template <>
+__device__ __forceinline__ float lds<float>(uint32_t a) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+template <>
+__device__ __forceinline__ float2 lds<float2>(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+    return v;
+}
+template <>
+__device__ __forceinline__ float4 lds<float4>(uint32_t a) {
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
     return v;
 }
-/* v = shared float at a where pred != 0 (a predicated load: no branch) */
-__device__ __forceinline__ void lds1_if(float &v, uint32_t a, uint32_t pred) {
+template <>
+__device__ __forceinline__ double lds<double>(uint32_t a) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+template <>
+__device__ __forceinline__ double2 lds<double2>(uint32_t a) {
+    double2 v;
+    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts(uint32_t a, float v) {
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void sts(uint32_t a, const float2 &v) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void sts(uint32_t a, const float4 &v) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+__device__ __forceinline__ void sts(uint32_t a, double v) {
+    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void sts(uint32_t a, const double2 &v) {
+    asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+/* v = shared value at a where pred != 0 (a predicated load: no branch) */
+__device__ __forceinline__ void lds_if(float &v, uint32_t a, uint32_t pred) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}"
                  : "+f"(v)
                  : "r"(a), "r"(pred));
 }
-__device__ __forceinline__ void sts4(uint32_t a, const float4 &v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                 : "memory");
+__device__ __forceinline__ void lds_if(double &v, uint32_t a, uint32_t pred) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f64 %0, [%1];\n\t}"
+                 : "+d"(v)
+                 : "r"(a), "r"(pred));
 }
 
+/* the sites of 1, 2 or 4 consecutive positions, by their count */
+template <typename T, int N>
+struct Part;
+template <>
+struct Part<float, 1> { using V = float; };
+template <>
+struct Part<float, 2> { using V = float2; };
+template <>
+struct Part<float, 4> { using V = float4; };
+template <>
+struct Part<double, 1> { using V = double; };
+template <>
+struct Part<double, 2> { using V = double2; };
+__device__ __forceinline__ float first(float v) { return v; }
+__device__ __forceinline__ float first(const float2 &v) { return v.x; }
+__device__ __forceinline__ float first(const float4 &v) { return v.x; }
+__device__ __forceinline__ double first(double v) { return v; }
+__device__ __forceinline__ double first(const double2 &v) { return v.x; }
+__device__ __forceinline__ float last(float v) { return v; }
+__device__ __forceinline__ float last(const float2 &v) { return v.y; }
+__device__ __forceinline__ float last(const float4 &v) { return v.w; }
+__device__ __forceinline__ double last(double v) { return v; }
+__device__ __forceinline__ double last(const double2 &v) { return v.y; }
 
-/* Packed constants of the static float update (a = 1). */
-struct Pk {
+/* One leapfrog step on the static background: pi' = pi + dt F(phi), phi' =
+ * phi + dt pi' (bubble.cpp:716-743, 853-856, 867-870 with a = 1), for the
+ * sites c of a row with its neighbour rows um / up along axis 1 and im / ip
+ * along axis 0 and the sites left / right of it along axis 2 -- the results
+ * of the single-step kernel bit for bit. */
+template <typename T, int BY>
+struct Step;
+
+/* float: packed pairs (f32x2); one site: both halves of a pair carry it (each
+ * half is rounded on its own) */
+template <int BY>
+struct Step<float, BY> {
     F2 idx2, dt, nc2, c3, nc4;
-};
-
-/* One 16-byte vector (sites kk .. kk+3 of one row) of one leapfrog step on the
- * static background: pi' = pi + dt F(phi), phi' = phi + dt pi' (bubble.cpp:
- * 716-743, 853-856, 867-870 with a = 1), as two packed pairs -- the results of
- * the single-step kernel's packed path bit for bit. */
-/* One packed pair of sites (two neighbours along axis 2): the force with the
- * periodic Laplacian and V'(phi), the kick and the drift. */
-__device__ __forceinline__ void upd_pair(const Pk &K, F2 cc, F2 umm, F2 upp, F2 imm, F2 ipp, F2 kmm, F2 kpp, F2 pp,
-                                         F2 &phi2, F2 &pi2) {
-    const F2 two = f2_add(cc, cc);
-    const F2 t0 = f2_add(f2_sub(ipp, two), imm);
-    const F2 t1 = f2_add(f2_sub(upp, two), umm);
-    const F2 t2 = f2_add(f2_sub(kpp, two), kmm);
-    const F2 lap = f2_add(f2_add(t0, t1), t2);
-    /* -V'(f)/f = -(c2 + f (-c3 + f c4)) with every operand negated: the
-     * exact negation of the one-step kernel's rounded h (round to nearest
-     * is symmetric); with a^(d-2) = a^d = 1 the force fma(1 lap, 1/dx^2,
-     * -1 (f h)) is then fma(lap, 1/dx^2, f (-h)), bit for bit */
-    const F2 nh = f2_fma(cc, f2_fma(cc, K.nc4, K.c3), K.nc2);
-    const F2 force = f2_fma(lap, K.idx2, f2_mul(cc, nh));
-    pi2 = f2_fma(K.dt, force, pp);
-    phi2 = f2_fma(K.dt, pi2, cc);
-}
-
-__device__ __forceinline__ void update4(const Pk &K, const float4 c, const float4 um, const float4 up, const float4 im,
-                                        const float4 ip, float left, float right, const float4 pv, float4 &phi_n,
-                                        float4 &pi_n) {
-    const F2 c01 = f2_pack(c.x, c.y), c23 = f2_pack(c.z, c.w);
-    const F2 km01 = f2_pack(left, c.x), mid = f2_pack(c.y, c.z), kp23 = f2_pack(c.w, right);
-    F2 phi01, pi01, phi23, pi23;
-    upd_pair(K, c01, f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y), f2_pack(ip.x, ip.y), km01, mid,
-             f2_pack(pv.x, pv.y), phi01, pi01);
-    upd_pair(K, c23, f2_pack(um.z, um.w), f2_pack(up.z, up.w), f2_pack(im.z, im.w), f2_pack(ip.z, ip.w), mid, kp23,
-             f2_pack(pv.z, pv.w), phi23, pi23);
-    phi_n = make_float4(f2_lo(phi01), f2_hi(phi01), f2_lo(phi23), f2_hi(phi23));
-    pi_n = make_float4(f2_lo(pi01), f2_hi(pi01), f2_lo(pi23), f2_hi(pi23));
-}
-
-/* The halo rows' share of a thread: HW consecutive sites of a row (HW = 1, 2
- * or 4), as float, float2 or float4, with shared-memory loads and stores of
- * that width, and the update of those sites (the same packed pairs). */
-template <int HW>
-struct Hv;
-template <>
-struct Hv<4> {
-    using T = float4;
-    static __device__ __forceinline__ T ld(uint32_t a) { return lds4(a); }
-    static __device__ __forceinline__ void st(uint32_t a, const T &v) { sts4(a, v); }
-    static __device__ __forceinline__ float first(const T &v) { return v.x; }
-    static __device__ __forceinline__ float last(const T &v) { return v.w; }
-    static __device__ __forceinline__ void update(const Pk &K, const T &c, const T &um, const T &up, const T &im,
-                                                  const T &ip, float left, float right, const T &pv, T &phi, T &pi) {
-        update4(K, c, um, up, im, ip, left, right, pv, phi, pi);
+    __device__ __forceinline__ explicit Step(const StepConst &k)
+        : idx2(f2_splat(k.inv_dx2f)), dt(f2_splat(k.dtf)), nc2(f2_splat(-k.c2f)), c3(f2_splat(k.c3f)),
+          nc4(f2_splat(-k.c4f)) {}
+    __device__ __forceinline__ void pair(F2 cc, F2 umm, F2 upp, F2 imm, F2 ipp, F2 kmm, F2 kpp, F2 pp, F2 &phi2,
+                                         F2 &pi2) const {
+        const F2 two = f2_add(cc, cc);
+        const F2 t0 = f2_add(f2_sub(ipp, two), imm);
+        const F2 t1 = f2_add(f2_sub(upp, two), umm);
+        const F2 t2 = f2_add(f2_sub(kpp, two), kmm);
+        const F2 lap = f2_add(f2_add(t0, t1), t2);
+        /* -V'(f)/f = -(c2 + f (-c3 + f c4)) with every operand negated: the
+         * exact negation of the one-step kernel's rounded h (round to nearest
+         * is symmetric); with a^(d-2) = a^d = 1 the force fma(1 lap, 1/dx^2,
+         * -1 (f h)) is then fma(lap, 1/dx^2, f (-h)), bit for bit */
+        const F2 nh = f2_fma(cc, f2_fma(cc, nc4, c3), nc2);
+        const F2 force = f2_fma(lap, idx2, f2_mul(cc, nh));
+        pi2 = f2_fma(dt, force, pp);
+        phi2 = f2_fma(dt, pi2, cc);
     }
-};
-template <>
-struct Hv<2> {
-    using T = float2;
-    static __device__ __forceinline__ T ld(uint32_t a) {
-        float2 v;
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-        return v;
+    __device__ __forceinline__ void operator()(const float4 &c, const float4 &um, const float4 &up, const float4 &im,
+                                               const float4 &ip, float left, float right, const float4 &pv,
+                                               float4 &phi, float4 &pi) const {
+        const F2 mid = f2_pack(c.y, c.z);
+        F2 phi01, pi01, phi23, pi23;
+        pair(f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y), f2_pack(ip.x, ip.y),
+             f2_pack(left, c.x), mid, f2_pack(pv.x, pv.y), phi01, pi01);
+        pair(f2_pack(c.z, c.w), f2_pack(um.z, um.w), f2_pack(up.z, up.w), f2_pack(im.z, im.w), f2_pack(ip.z, ip.w),
+             mid, f2_pack(c.w, right), f2_pack(pv.z, pv.w), phi23, pi23);
+        phi = make_float4(f2_lo(phi01), f2_hi(phi01), f2_lo(phi23), f2_hi(phi23));
+        pi = make_float4(f2_lo(pi01), f2_hi(pi01), f2_lo(pi23), f2_hi(pi23));
     }
-    static __device__ __forceinline__ void st(uint32_t a, const T &v) {
-        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
-    }
-    static __device__ __forceinline__ float first(const T &v) { return v.x; }
-    static __device__ __forceinline__ float last(const T &v) { return v.y; }
-    static __device__ __forceinline__ void update(const Pk &K, const T &c, const T &um, const T &up, const T &im,
-                                                  const T &ip, float left, float right, const T &pv, T &phi, T &pi) {
+    __device__ __forceinline__ void operator()(const float2 &c, const float2 &um, const float2 &up, const float2 &im,
+                                               const float2 &ip, float left, float right, const float2 &pv,
+                                               float2 &phi, float2 &pi) const {
         F2 p2, q2;
-        upd_pair(K, f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y),
-                 f2_pack(ip.x, ip.y), f2_pack(left, c.x), f2_pack(c.y, right), f2_pack(pv.x, pv.y), p2, q2);
+        pair(f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y), f2_pack(ip.x, ip.y),
+             f2_pack(left, c.x), f2_pack(c.y, right), f2_pack(pv.x, pv.y), p2, q2);
         phi = make_float2(f2_lo(p2), f2_hi(p2));
         pi = make_float2(f2_lo(q2), f2_hi(q2));
     }
-};
-template <>
-struct Hv<1> {
-    using T = float;
-    static __device__ __forceinline__ T ld(uint32_t a) {
-        float v;
-        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-        return v;
-    }
-    static __device__ __forceinline__ void st(uint32_t a, const T &v) {
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-    }
-    static __device__ __forceinline__ float first(const T &v) { return v; }
-    static __device__ __forceinline__ float last(const T &v) { return v; }
-    /* one site: both halves of the pair carry it (each half is rounded on its own) */
-    static __device__ __forceinline__ void update(const Pk &K, const T &c, const T &um, const T &up, const T &im,
-                                                  const T &ip, float left, float right, const T &pv, T &phi, T &pi) {
+    __device__ __forceinline__ void operator()(float c, float um, float up, float im, float ip, float left,
+                                               float right, float pv, float &phi, float &pi) const {
         F2 p2, q2;
-        upd_pair(K, f2_splat(c), f2_splat(um), f2_splat(up), f2_splat(im), f2_splat(ip), f2_splat(left),
-                 f2_splat(right), f2_splat(pv), p2, q2);
+        pair(f2_splat(c), f2_splat(um), f2_splat(up), f2_splat(im), f2_splat(ip), f2_splat(left), f2_splat(right),
+             f2_splat(pv), p2, q2);
         phi = f2_lo(p2);
         pi = f2_lo(q2);
+    }
+};
+
+/* double: the single-step kernel's rounded operations in its order, without
+ * its products with a^(d-2) = a^d = 1 (exact) */
+template <int BY>
+struct Step<double, BY> {
+    const StepConst &k;
+    __device__ __forceinline__ explicit Step(const StepConst &kk) : k(kk) {}
+    __device__ __forceinline__ void operator()(double c, double um, double up, double im, double ip, double left,
+                                               double right, double pv, double &phi, double &pi) const {
+        using A = Ar<double>;
+        const double two = A::add(c, c);
+        const double t0 = A::add(A::sub(ip, two), im);
+        const double t1 = A::add(A::sub(up, two), um);
+        const double t2 = A::add(A::sub(right, two), left);
+        const double lap = A::add(A::add(t0, t1), t2);
+        pi = A::add(pv, A::mul(k.dt, A::sub(over_dx2<BY>(k, lap), dV<double>(k, c))));
+        phi = A::add(c, A::mul(k.dt, pi));
+    }
+    __device__ __forceinline__ void operator()(const double2 &c, const double2 &um, const double2 &up,
+                                               const double2 &im, const double2 &ip, double left, double right,
+                                               const double2 &pv, double2 &phi, double2 &pi) const {
+        (*this)(c.x, um.x, up.x, im.x, ip.x, left, c.y, pv.x, phi.x, pi.x);
+        (*this)(c.y, um.y, up.y, im.y, ip.y, c.x, right, pv.y, phi.y, pi.y);
     }
 };
 
@@ -186,8 +245,9 @@ struct Hv<1> {
  *   z, zz     level-1 pi at planes m', m' + 1.
  * The halo rows (j0 - 1, j0 + tj) are updated at level 1 only; a thread's
  * share of them keeps only x_m, x_c. */
+template <typename V>
 struct Slot {
-    float4 x_m, x_c, y_m, y_c, y_p, z, zz;
+    V x_m, x_c, y_m, y_c, y_p, z, zz;
 };
 
 /* Two leapfrog steps per pass (see the file comment). Thread c owns the tile
@@ -207,12 +267,13 @@ struct Slot {
  * ends with one barrier of all threads; plane g's stage is free once round
  * g + 1 has ended, so at the start of round g thread 0 issues the copies of
  * planes up to g + nstage - 2 (no other wait). */
-template <int HW>
+template <typename T, int BY, int HW, bool WHOLE>
 __global__ void __launch_bounds__(TB_MAXT, 1)
-    k_step3_t2(StepConst k, int tj, int nstage, int parts, const float *__restrict__ phi_in,
-               const float *__restrict__ pi_in, float *__restrict__ phi_out, float *__restrict__ pi_out,
-               DevState *st) {
-    constexpr int W = 4;
+    k_step3_t2(StepConst k, int tj, int nstage, int parts, const T *__restrict__ phi_in, const T *__restrict__ pi_in,
+               T *__restrict__ phi_out, T *__restrict__ pi_out, DevState *st) {
+    using V = typename Vec<T>::V;
+    constexpr int W = Vec<T>::W;
+    constexpr uint32_t ES = sizeof(T);
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ int abort_flag;
     __shared__ int item_q[TB_IQ];
@@ -221,15 +282,15 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     const int R0 = tj + 4;                 /* input phi rows: j0 - 2 .. j0 + tj + 1 */
     const int R0p = tj + 2;                /* input pi rows: j0 - 1 .. j0 + tj */
     const int R1 = tj + 2;                 /* level-1 phi rows: j0 - 1 .. j0 + tj */
-    const int stage_n = (R0 + R0p) * n;    /* floats per input stage */
-    const int slot_n = R1 * n;             /* floats per level-1 slot */
+    const int stage_n = (R0 + R0p) * n;    /* elements per input stage */
+    const int slot_n = R1 * n;             /* elements per level-1 slot */
     uint64_t *full = reinterpret_cast<uint64_t *>(smraw);
-    float *ring = reinterpret_cast<float *>(smraw + TB_HDR);
-    float *l1 = ring + (size_t)nstage * stage_n;
+    T *ring = reinterpret_cast<T *>(smraw + TB_HDR);
+    T *l1 = ring + (size_t)nstage * stage_n;
 
-    const int ntiles = n / tj;
+    const int ntiles = (n + tj - 1) / tj;
     const int items = ntiles * parts;
-    const size_t row_bytes = (size_t)n * sizeof(float);
+    const size_t row_bytes = (size_t)n * sizeof(T);
     const size_t plane = (size_t)n * n;
     const uint32_t tx_bytes = (uint32_t)((size_t)(R0 + R0p) * row_bytes);
     const int lane = threadIdx.x & 31;
@@ -245,10 +306,11 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      *      producer's item j is published in item_q[j % TB_IQ] before its
      *      first plane is issued ---- */
     int pr_j = 0, pr_it = -1, pr_pl = 0, pr_p1 = 0;              /* producer: item, next plane */
-    /* the item's source rows (periodic), as element offsets within a plane:
-     * phi rows j0 - 2, j0 - 1, j0 .. j0 + tj - 1, j0 + tj, j0 + tj + 1; pi rows
-     * j0 - 1, j0 .. j0 + tj - 1, j0 + tj */
-    __shared__ size_t pr_r[6];   /* thread 0's only: kept out of the registers */
+    /* the item's source rows, as element offsets within a plane and counts of
+     * rows: phi rows j0 - 2 .. j0 + tj + 1 and pi rows j0 - 1 .. j0 + tj, each from
+     * its start up to the lattice's last row, then the rest from row 0 */
+    __shared__ size_t pr_r[2];   /* thread 0's only: kept out of the registers */
+    __shared__ int pr_c[2];
     long long issued = 0;                                        /* planes issued so far */
     int is_stage = 0;                                            /* its stage: issued mod nstage */
     bool pr_done = false;
@@ -268,28 +330,28 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         pr_pl = p0 - 2;
         pr_p1 = p1;
         const int j0 = t * tj;
-        const int rows[6] = {(j0 - 2 + n) % n, (j0 - 1 + n) % n, j0, (j0 + tj) % n, (j0 + tj + 1) % n, 0};
-        for (int e = 0; e < 6; ++e) pr_r[e] = (size_t)rows[e] * n;
+        const int r0 = (j0 - 2 + n) % n, r1 = (j0 - 1 + n) % n;
+        pr_r[0] = (size_t)r0 * n;
+        pr_r[1] = (size_t)r1 * n;
+        pr_c[0] = min(R0, n - r0);
+        pr_c[1] = min(R0p, n - r1);
     };
     auto issue_upto = [&](long long last) {
         while (!pr_done && issued <= last) {
             const int s = is_stage;
             const int pw = pr_pl < 0 ? pr_pl + n : (pr_pl >= n ? pr_pl - n : pr_pl);
-            float *dst = ring + (size_t)s * stage_n;
-            float *dpi = dst + (size_t)R0 * n;
-            const float *gphi = phi_in + (size_t)pw * plane;
-            const float *gpi = pi_in + (size_t)pw * plane;
+            T *dst = ring + (size_t)s * stage_n;
+            T *dpi = dst + (size_t)R0 * n;
+            const T *gphi = phi_in + (size_t)pw * plane;
+            const T *gpi = pi_in + (size_t)pw * plane;
             const uint32_t rb = (uint32_t)row_bytes;
             fence_proxy_async();
             mbar_arrive_expect_tx(&full[s], tx_bytes);
-            bulk_g2s(dst, gphi + pr_r[0], rb, &full[s]);
-            bulk_g2s(dst + n, gphi + pr_r[1], rb, &full[s]);
-            bulk_g2s(dst + (size_t)2 * n, gphi + pr_r[2], (uint32_t)tj * rb, &full[s]);
-            bulk_g2s(dst + (size_t)(2 + tj) * n, gphi + pr_r[3], rb, &full[s]);
-            bulk_g2s(dst + (size_t)(3 + tj) * n, gphi + pr_r[4], rb, &full[s]);
-            bulk_g2s(dpi, gpi + pr_r[1], rb, &full[s]);
-            bulk_g2s(dpi + n, gpi + pr_r[2], (uint32_t)tj * rb, &full[s]);
-            bulk_g2s(dpi + (size_t)(1 + tj) * n, gpi + pr_r[3], rb, &full[s]);
+            const int c0 = pr_c[0], c1 = pr_c[1];
+            bulk_g2s(dst, gphi + pr_r[0], (uint32_t)c0 * rb, &full[s]);
+            if (c0 < R0) bulk_g2s(dst + (size_t)c0 * n, gphi, (uint32_t)(R0 - c0) * rb, &full[s]);
+            bulk_g2s(dpi, gpi + pr_r[1], (uint32_t)c1 * rb, &full[s]);
+            if (c1 < R0p) bulk_g2s(dpi + (size_t)c1 * n, gpi, (uint32_t)(R0p - c1) * rb, &full[s]);
             ++issued;
             if (++is_stage == nstage) is_stage = 0;
             if (++pr_pl > pr_p1 + 1) next_item();
@@ -309,42 +371,55 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     }
     __syncthreads();
 
-    Pk K;
-    K.idx2 = f2_splat(k.inv_dx2f);
-    K.dt = f2_splat(k.dtf);
-    K.nc2 = f2_splat(-k.c2f);
-    K.c3 = f2_splat(k.c3f);
-    K.nc4 = f2_splat(-k.c4f);
+    const Step<T, BY> step(k);
     /* the positions as offsets r1 n + kk in an array of level-1 rows (row r1,
      * first site kk; rows hold n = W nvr sites, so tile position u sits at
-     * n + W u): tile slot s at off0 + s W NT, the halo slot at offh */
-    const int off0 = n + W * threadIdx.x, slot_step = W * NT;
-    using H = Hv<HW>;
-    using HT = typename H::T;
-    const bool has_h = HW * (int)threadIdx.x < 2 * n;
-    const int fh = HW * threadIdx.x;                        /* first halo site, counted over both rows */
+     * n + W u): tile slot s at off0 + s W NT, the halo slot at offh. Where the
+     * tile's positions are no multiple of the threads (!WHOLE), the spare ones
+     * repeat the last position and store nothing. */
+    const int npos = tj * (n / W), slot_step = W * NT;
+    int offs[TB_NTS];
+    bool own[TB_NTS];
+#pragma unroll
+    for (int s = 0; s < TB_NTS; ++s) {
+        const int u = threadIdx.x + s * NT;
+        own[s] = WHOLE || u < npos;
+        offs[s] = n + W * (own[s] ? u : npos - 1);
+    }
+    using HT = typename Part<T, HW>::V;
+    /* whole warps take part in the halo rows (they shuffle) */
+    const bool has_h = HW * (int)(WHOLE ? threadIdx.x : threadIdx.x & ~31) < 2 * n;
+    const bool own_h = HW * (int)threadIdx.x < 2 * n;
+    const int fh = own_h ? HW * (int)threadIdx.x : 2 * n - HW;   /* first halo site, counted over both rows */
     const int offh = fh + (fh < n ? 0 : tj * n);
-    const uint32_t first_lane = lane == 0, last_lane = lane == 31;
-    /* every slot of a thread starts at the same site of its row (the slots are
-     * whole rows apart: tj is even), kk = W threadIdx.x mod n; the periodic
-     * wrap of its axis-2 neighbours, for the lanes that read them */
-    const int kk_own = (W * threadIdx.x) % n;
-    const int ladj = kk_own == 0 ? n : 0, radj = kk_own + W == n ? -n : 0;
     /* the axis-2 neighbours of the vector at shared byte address a: from the
-     * neighbouring lanes, the warp's end lanes from the row */
-    const int ladj_b = 4 * (ladj - 1), radj_b = 4 * (radj + W);
+     * neighbouring lanes, at the warp's ends and the row's ends from the row
+     * (periodic). WHOLE: every slot of a thread starts at the same site of its
+     * row (the slots are whole rows apart) and a row is whole warps. */
+    uint32_t from_l[TB_NTS], from_r[TB_NTS];
+    int ladj_b[TB_NTS], radj_b[TB_NTS];
+#pragma unroll
+    for (int s = 0; s < TB_NTS; ++s) {
+        const int kk = offs[s] % n;
+        from_l[s] = lane == 0 || (!WHOLE && kk == 0);
+        from_r[s] = lane == 31 || (!WHOLE && kk + W == n);
+        ladj_b[s] = (int)ES * ((kk == 0 ? n : 0) - 1);
+        radj_b[s] = (int)ES * ((kk + W == n ? -n : 0) + W);
+    }
     /* the same for the halo share (first site kk_h of its row, HW sites) */
     const int kk_h = fh % n;
-    const int ladjh_b = 4 * ((kk_h == 0 ? n : 0) - 1), radjh_b = 4 * ((kk_h + HW == n ? -n : 0) + HW);
-    auto sides = [&](const float4 &c, uint32_t a, float &left, float &right) {
-        left = __shfl_up_sync(0xffffffffu, c.w, 1);
-        right = __shfl_down_sync(0xffffffffu, c.x, 1);
-        lds1_if(left, a + ladj_b, first_lane);
-        lds1_if(right, a + radj_b, last_lane);
+    const uint32_t from_lh = lane == 0 || (!WHOLE && kk_h == 0), from_rh = lane == 31 || (!WHOLE && kk_h + HW == n);
+    const int ladjh_b = (int)ES * ((kk_h == 0 ? n : 0) - 1), radjh_b = (int)ES * ((kk_h + HW == n ? -n : 0) + HW);
+    auto sides = [&](const V &c, uint32_t a, int s, T &left, T &right) {
+        const int q = WHOLE ? 0 : s;
+        left = __shfl_up_sync(0xffffffffu, last(c), 1);
+        right = __shfl_down_sync(0xffffffffu, first(c), 1);
+        lds_if(left, a + ladj_b[q], from_l[q]);
+        lds_if(right, a + radj_b[q], from_r[q]);
     };
     const uint32_t ring_a = smem_u32(ring), l1_a = smem_u32(l1);
-    const uint32_t stage_b = 4u * (uint32_t)stage_n, slot_b = 4u * (uint32_t)slot_n, nb = 4u * (uint32_t)n;
-    const uint32_t pi_b = 4u * (uint32_t)(R0 * n);
+    const uint32_t stage_b = ES * (uint32_t)stage_n, slot_b = ES * (uint32_t)slot_n, nb = ES * (uint32_t)n;
+    const uint32_t pi_b = ES * (uint32_t)(R0 * n);
     /* the stage and phase parity of round g's plane, advanced once per round */
     int gs = 0, gs_prev = 0;
     uint32_t gph = 0u;
@@ -369,8 +444,9 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         if (!any_bad && threadIdx.x == 0) issue_upto(g + nstage - 1);
         return any_bad;
     };
-    Slot sl[TB_NTS];
+    Slot<V> sl[TB_NTS];
     HT hxm, hxc;
+    auto at = [&](int s) { return WHOLE ? offs[0] + s * slot_step : offs[s]; };
     long long g = 0;     /* the round: index of the input plane it waits for */
     bool bad = false;
     for (int j = 0;; ++j) {
@@ -379,12 +455,16 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         int t, p0, p1;
         item_of(it, t, p0, p1);
         const int j0 = t * tj;
+        /* the slots whose level-2 row is the lattice's (the last tile may hang over) */
+        bool keep[TB_NTS];
+#pragma unroll
+        for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own[s] && j0 * n + offs[s] - n < n * n);
         /* input planes p0 - 2 and p0 - 1: this thread's phi into the register queues */
         if (!bad && acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
 #pragma unroll
-            for (int s = 0; s < TB_NTS; ++s) sl[s].x_m = lds4(S + 4u * (off0 + s * slot_step));
-            if (has_h) hxm = H::ld(S + 4u * offh);
+            for (int s = 0; s < TB_NTS; ++s) sl[s].x_m = lds<V>(S + ES * at(s));
+            if (has_h) hxm = lds<HT>(S + ES * offh);
         } else {
             bad = true;
         }
@@ -394,8 +474,8 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         if (!bad && acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
 #pragma unroll
-            for (int s = 0; s < TB_NTS; ++s) sl[s].x_c = lds4(S + 4u * (off0 + s * slot_step));
-            if (has_h) hxc = H::ld(S + 4u * offh);
+            for (int s = 0; s < TB_NTS; ++s) sl[s].x_c = lds<V>(S + ES * at(s));
+            if (has_h) hxc = lds<HT>(S + ES * offh);
         } else {
             bad = true;
         }
@@ -412,17 +492,17 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                 const uint32_t S0 = ring_a + gs_prev * stage_b;   /* plane q - 1 */
                 const uint32_t D1 = l1_a + ((q - p0) & 1) * slot_b;   /* level-1 plane q - 1 */
                 /* level 1 at plane q - 1, at one position with input queue (xm, xc) */
-                auto level1 = [&](float4 &xm, float4 &xc, int off, float4 &phi1, float4 &pi1) {
+                auto level1 = [&](V &xm, V &xc, int s, V &phi1, V &pi1) {
                     /* input phi row 0 is level-1 row -1: the centre sits at n + off */
-                    const uint32_t ob = 4u * (uint32_t)off;
-                    const float4 x_p = lds4(Sn + nb + ob);
-                    const float4 um = lds4(S0 + ob);
-                    const float4 up = lds4(S0 + 2u * nb + ob);
-                    const float4 pv = lds4(S0 + pi_b + ob);
-                    float left, right;
-                    sides(xc, S0 + nb + ob, left, right);
-                    update4(K, xc, um, up, xm, x_p, left, right, pv, phi1, pi1);
-                    sts4(D1 + ob, phi1);
+                    const uint32_t ob = ES * (uint32_t)at(s);
+                    const V x_p = lds<V>(Sn + nb + ob);
+                    const V um = lds<V>(S0 + ob);
+                    const V up = lds<V>(S0 + 2u * nb + ob);
+                    const V pv = lds<V>(S0 + pi_b + ob);
+                    T left, right;
+                    sides(xc, S0 + nb + ob, s, left, right);
+                    step(xc, um, up, xm, x_p, left, right, pv, phi1, pi1);
+                    if (own[s]) sts(D1 + ob, phi1);
                     xm = xc;
                     xc = x_p;
                 };
@@ -432,47 +512,48 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                 const uint32_t L0 = l1_a + ((m2 - p0 + 1) & 1) * slot_b;
                 /* global row j0 - 1 + r1 of plane m2: the tile position's offset from row j0 - 1 */
                 const size_t gbase = ((size_t)m2 * n + (size_t)j0) * n - (size_t)n;
-                auto level2 = [&](Slot &x, int off) {
-                    const uint32_t ob = L0 + 4u * (uint32_t)off;
-                    const float4 um = lds4(ob - nb);
-                    const float4 up = lds4(ob + nb);
-                    float left, right;
-                    sides(x.y_c, ob, left, right);
-                    float4 phi2, pi2;
-                    update4(K, x.y_c, um, up, x.y_m, x.y_p, left, right, x.z, phi2, pi2);
-                    *reinterpret_cast<float4 *>(phi_out + (gbase + off)) = phi2;
-                    *reinterpret_cast<float4 *>(pi_out + (gbase + off)) = pi2;
+                auto level2 = [&](Slot<V> &x, int s) {
+                    const uint32_t ob = L0 + ES * (uint32_t)at(s);
+                    const V um = lds<V>(ob - nb);
+                    const V up = lds<V>(ob + nb);
+                    T left, right;
+                    sides(x.y_c, ob, s, left, right);
+                    V phi2, pi2;
+                    step(x.y_c, um, up, x.y_m, x.y_p, left, right, x.z, phi2, pi2);
+                    if (keep[s]) {
+                        *reinterpret_cast<V *>(phi_out + (gbase + at(s))) = phi2;
+                        *reinterpret_cast<V *>(pi_out + (gbase + at(s))) = pi2;
+                    }
                 };
                 /* per tile position: level 1 at plane q - 1, then level 2 at plane q - 2,
                  * which needs the position's own level-1 plane q - 1 just computed */
 #pragma unroll
                 for (int s = 0; s < TB_NTS; ++s) {
-                    Slot &x = sl[s];
-                    const int off = off0 + s * slot_step;
-                    float4 phi1, pi1;
-                    level1(x.x_m, x.x_c, off, phi1, pi1);
+                    Slot<V> &x = sl[s];
+                    V phi1, pi1;
+                    level1(x.x_m, x.x_c, s, phi1, pi1);
                     x.y_m = x.y_c;
                     x.y_c = x.y_p;
                     x.y_p = phi1;
                     x.z = x.zz;
                     x.zz = pi1;
-                    if (m2 >= p0) level2(x, off);
+                    if (m2 >= p0) level2(x, s);
                 }
                 if (has_h) {
                     /* level 1 at plane q - 1 on the halo share */
-                    const uint32_t ob = 4u * (uint32_t)offh;
-                    const HT xp = H::ld(Sn + nb + ob);
-                    const HT um = H::ld(S0 + ob);
-                    const HT up = H::ld(S0 + 2u * nb + ob);
-                    const HT pv = H::ld(S0 + pi_b + ob);
+                    const uint32_t ob = ES * (uint32_t)offh;
+                    const HT xp = lds<HT>(Sn + nb + ob);
+                    const HT um = lds<HT>(S0 + ob);
+                    const HT up = lds<HT>(S0 + 2u * nb + ob);
+                    const HT pv = lds<HT>(S0 + pi_b + ob);
                     const uint32_t a = S0 + nb + ob;
-                    float left = __shfl_up_sync(0xffffffffu, H::last(hxc), 1);
-                    float right = __shfl_down_sync(0xffffffffu, H::first(hxc), 1);
-                    lds1_if(left, a + ladjh_b, first_lane);
-                    lds1_if(right, a + radjh_b, last_lane);
+                    T left = __shfl_up_sync(0xffffffffu, last(hxc), 1);
+                    T right = __shfl_down_sync(0xffffffffu, first(hxc), 1);
+                    lds_if(left, a + ladjh_b, from_lh);
+                    lds_if(right, a + radjh_b, from_rh);
                     HT phi1, pi1;
-                    H::update(K, hxc, um, up, hxm, xp, left, right, pv, phi1, pi1);
-                    H::st(D1 + ob, phi1);
+                    step(hxc, um, up, hxm, xp, left, right, pv, phi1, pi1);
+                    if (WHOLE || own_h) sts(D1 + ob, phi1);
                     hxm = hxc;
                     hxc = xp;
                 }
@@ -511,61 +592,58 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
 
 int sm_count();
 
-/* Threads of the two-step pass: TB_NTS tile positions each (tj rows of n / 4
- * vectors); 0 when that is not a whole number of warps or the halo rows'
- * 2 n / 4 positions outnumber the threads. */
-int step3tb_consumers(int n, int tj) {
-    const int v2 = tj * (n / 4);
-    if (v2 % (32 * TB_NTS) != 0 || v2 / TB_NTS < 2 * (n / 4)) return 0;
-    return v2 / TB_NTS;
-}
-
-/* Geometry of the two-step pass: float fields, d = 3, static background,
- * n a multiple of 128 (rows of a multiple of 32 vectors). TJ rows per tile:
- * the largest divisor of n (at most 32) whose shared memory -- 4 to 6 input
- * stages of (2 TJ + 6) rows and 2 level-1 planes of TJ + 2 rows -- fits the
- * 227 KB of one block per SM, with at most 16 warps (two tile positions
- * per thread): 8 rows at 512^3, 16 at 256^3. The number of plane
- * parts minimises whole rounds of items over the SMs times an item's
- * rounds (its planes plus two). */
+/* Geometry of the two-step pass (d = 3, static background, n a multiple of
+ * the 16-byte vector, rows of at least one warp: with shorter ones a round's
+ * latency is all there is, 100^3 in float 6.5 us per step against 6.7). A tile is TJ rows; its TJ n / W positions are two per
+ * thread, at most 512 threads (so TJ n <= 4096 floats or 2048 doubles), and
+ * the halo rows' 2 n / W positions are no more than the threads (TJ >= 4).
+ * Shared memory: 4 to 6 input stages of 2 TJ + 6 rows and 2 level-1 planes of
+ * TJ + 2 rows in the 227 KB of one block per SM. TJ and the plane parts P are
+ * those of the least modelled time: whole rounds of items over the SMs, times
+ * the planes an item streams (n / P and four beyond them), times a plane's
+ * time, 1 us (the chain of its loads, updates and barrier; 1.15 in general) and 0.036 us (float)
+ * or 0.05 us (double) per vector of a scheduler's warps (64^3 1.1 us a plane,
+ * 512^3 1.63, 256^3 in double 1.86). So 512^3 takes 9 parts in 4 rounds (198.6
+ * us per step; 16 parts in 7 rounds 213). Double needs dx^2 to divide in one
+ * or two operations (one step per pass otherwise). */
 bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage, size_t &smem, unsigned &grid,
                       int &parts) {
-    if (k.d != 3 || prec != P_FP32 || k.expanding || tl != 2) return false;
+    const int W = prec == P_FP64 ? 2 : 4;
     const int n = k.n;
-    if (n % 128 != 0 || n > 1024) return false;
-    const size_t esz = 4;
-    const size_t budget = 227 * 1024 - 1024;   /* dynamic share of 227 KB, room for the static variables */
-    tj = 0;
-    for (int t = 2; t <= 32 && t <= n; ++t) {
-        if (n % t != 0) continue;
-        const size_t stage = (size_t)(2 * t + 6) * n * esz;
-        const size_t lev = (size_t)2 * (t + 2) * n * esz;
-        const int nc = step3tb_consumers(n, t);
-        if (TB_HDR + lev + 4 * stage <= budget && nc > 0 && nc <= TB_MAXT) tj = t;
-    }
-    if (tj == 0) return false;
-    const size_t stage = (size_t)(2 * tj + 6) * n * esz;
-    const size_t lev = (size_t)2 * (tj + 2) * n * esz;
-    nstage = (int)((budget - TB_HDR - lev) / stage);
-    if (nstage > 6) nstage = 6;
-    smem = TB_HDR + (size_t)nstage * stage + lev;
-    const long long ntiles = n / tj;
+    if (k.d != 3 || k.expanding || tl != 2 || n % W != 0 || n / W < 32 || n > 1024) return false;
+    if (prec == P_FP64 && !k.dx2_pow2 && !k.dx2_pair) return false;
+    const size_t row = (size_t)n * (prec == P_FP64 ? 8 : 4);
+    const size_t budget = 227 * 1024 - 1024 - TB_HDR;   /* dynamic share of 227 KB, room for the static variables */
+    const int nv = n / W;
     const long long slots = sm_count();
-    double best = 1e300;
-    parts = 1;
-    for (int P = 1; P <= n / 4; ++P) {
-        const double per_item = (double)n / P + 2.0;
-        const long long rounds = (ntiles * P + slots - 1) / slots;
-        const double cost = (double)rounds * per_item;
-        if (cost < best - 1e-9) {
-            best = cost;
-            parts = P;
+    double best = 0.0;
+    for (int t = 4; t <= 32 && t * nv <= TB_NTS * TB_MAXT; ++t) {
+        const size_t stage = (size_t)(2 * t + 6) * row, lev = (size_t)2 * (t + 2) * row;
+        if (lev + 4 * stage > budget) break;
+        const long long ntiles = (n + t - 1) / t;
+        const int per_sched = (t * nv + 255) / 256;   /* warps per scheduler, two vectors each */
+        /* rows of whole warps in whole tiles save the masks and per-slot wraps (launch below) */
+        const bool whole = nv % 32 == 0 && n % t == 0 && t * nv % 64 == 0;
+        const double round = (whole ? 1.0 : 1.15) + (prec == P_FP64 ? 0.05 : 0.036) * (4.0 * per_sched + (2 * nv + 127) / 128);
+        for (long long w = 1; w <= 8; ++w) {
+            const long long P = std::min<long long>(w * slots / ntiles, n / 4);
+            if (P < 1) continue;
+            const long long waves = (ntiles * P + slots - 1) / slots;
+            const double cost = (double)waves * ((double)((n + P - 1) / P) + 4.0) * round;
+            if (best == 0.0 || cost < best) {
+                best = cost;
+                tj = t;
+                parts = (int)P;
+                nstage = (int)std::min<size_t>((budget - lev) / stage, 6);
+                smem = TB_HDR + (size_t)nstage * stage + lev;
+            }
         }
     }
+    if (best == 0.0) return false;
     const char *env = std::getenv("CB_STEP3TB_PARTS");
     if (env && std::atoi(env) >= 1 && std::atoi(env) <= n) parts = std::atoi(env);
-    const long long nitems = ntiles * parts;
-    grid = (unsigned)(nitems < slots ? nitems : slots);
+    const long long nitems = (long long)((n + tj - 1) / tj) * parts;
+    grid = (unsigned)std::min(nitems, slots);
     return true;
 }
 
@@ -575,14 +653,36 @@ cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *ph
     size_t smem;
     unsigned grid;
     if (!step3tb_geometry(k, prec, tl, tj, nstage, smem, grid, parts)) return cudaErrorInvalidValue;
-    const int nc = step3tb_consumers(k.n, tj);
-    /* the halo rows' 2 n sites over all threads where that is 1 or 2 sites each */
-    const int hw = (2 * k.n) % nc == 0 ? 2 * k.n / nc : 4;
-    auto fn = hw == 1 ? k_step3_t2<1> : (hw == 2 ? k_step3_t2<2> : k_step3_t2<4>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(fn, dim3(grid), dim3(nc), smem, s, k, tj, nstage, parts, (const float *)phi_in,
-                      (const float *)pi_in, (float *)phi_out, (float *)pi_out, st);
+    const int W = prec == P_FP64 ? 2 : 4;
+    const int npos = tj * (k.n / W);
+    const int nc = (npos + 64 - 1) / 64 * 32;
+    /* rows of whole warps, whole tiles, every thread two positions: the halo rows'
+     * 2 n sites then spread as 1, 2 (float: 4) per thread where that comes out even */
+    const bool whole = (k.n / W) % 32 == 0 && k.n % tj == 0 && npos == 2 * nc;
+    auto go = [&](auto t, auto by, auto hw, auto wh) -> cudaError_t {
+        using T = decltype(t);
+        auto fn = k_step3_t2<T, decltype(by)::value, decltype(hw)::value, decltype(wh)::value>;
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(fn, dim3(grid), dim3(nc), smem, s, k, tj, nstage, parts, (const T *)phi_in,
+                          (const T *)pi_in, (T *)phi_out, (T *)pi_out, st);
+    };
+    using std::integral_constant;
+    constexpr std::true_type yes{};
+    constexpr std::false_type no{};
+    constexpr integral_constant<int, 1> one{};
+    constexpr integral_constant<int, 2> two{};
+    constexpr integral_constant<int, 4> four{};
+    if (prec != P_FP64) {
+        constexpr integral_constant<int, BY_MUL> mul{};
+        if (!whole) return go(0.f, mul, four, no);
+        return 2 * k.n == nc ? go(0.f, mul, one, yes) : k.n == nc ? go(0.f, mul, two, yes) : go(0.f, mul, four, yes);
+    }
+    auto doubles = [&](auto by) {
+        if (!whole) return go(0.0, by, two, no);
+        return 2 * k.n == nc ? go(0.0, by, one, yes) : go(0.0, by, two, yes);
+    };
+    return k.dx2_pow2 ? doubles(integral_constant<int, BY_MUL>{}) : doubles(integral_constant<int, BY_PAIR>{});
 }
 
 }  // namespace cb
