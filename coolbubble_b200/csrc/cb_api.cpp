@@ -136,6 +136,7 @@ StepConst make_const(const cb_params *p) {
     k.nj = p->d >= 2 ? p->n_grids : 1;
     k.nk = p->n_grids;
     k.cz = 32;
+    k.pitch = run_pitch(p->d, p->n_grids, p->precision == CB_FP64 ? P_FP64 : P_FP32);
     k.dt = p->dt;
     const double cc = p->c;
     k.c2 = 2 * cc;               /* bubble.cpp:76: 2*cc*pow(phi,1) */
@@ -294,7 +295,7 @@ int alloc_handle(const cb_params *p, cb_handle **out) {
     keep_released_memory();
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { int r = cuda_fail(nullptr, e, "creating a stream"); delete h; return r; }
-    const size_t bytes = h->N * h->esz;
+    const size_t bytes = field_elems(h->k) * h->esz;
     /* stream-ordered allocations: creating and releasing a run never makes the
      * whole device wait (a serving loop creates and retires runs while others step) */
     auto dalloc = [&](void **ptr, size_t b) -> bool {
@@ -341,12 +342,48 @@ void destroy_handle(cb_handle *h) {
     delete h;
 }
 
+/* Elements of the staging buffer that padded fields go through (a lattice's
+ * worth would not fit beside the largest ones). */
+constexpr size_t STAGED_ELEMS = size_t(1) << 26;
+
+/* Download a field of padded rows into dense host memory of the given type;
+ * waits for each piece. */
+cudaError_t download_padded(cb_handle *h, const void *src, int to_prec, void *dst, int &status) {
+    const size_t n = (size_t)h->p.n_grids, pitch = (size_t)h->k.pitch, rows = h->N / n;
+    const size_t osz = to_prec == P_FP64 ? sizeof(double) : sizeof(float);
+    const size_t most = std::max<size_t>(1, std::min(rows, STAGED_ELEMS / n));
+    if ((status = ensure_tmp(h, most * n * osz)) != CB_OK) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
+    for (size_t at = 0; at < rows && e == cudaSuccess; at += most) {
+        const size_t m = std::min(most, rows - at);
+        e = launch_repitch(h->prec, to_prec, (const char *)src + at * pitch * h->esz, pitch, h->tmp, n, (int)n, m,
+                           h->stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync((char *)dst + at * n * osz, h->tmp, m * n * osz, cudaMemcpyDeviceToHost, h->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    }
+    return e;
+}
+
 /* Upload n doubles into a field buffer of the handle's precision. For FP32C
  * the doubles go to the device as they are (straight from the caller's,
  * possibly pinned, buffer) and are rounded to float there. */
 int upload_field(cb_handle *h, void *dst, const double *src) {
-    cudaError_t e;
-    if (h->prec == P_FP64) {
+    cudaError_t e = cudaSuccess;
+    const size_t n = (size_t)h->p.n_grids, pitch = (size_t)h->k.pitch, rows = h->N / n;
+    if (pitch != n) {
+        /* padded rows: dense pieces through a bounded staging buffer */
+        const size_t most = std::max<size_t>(1, std::min(rows, STAGED_ELEMS / n));
+        int r = ensure_tmp(h, most * n * sizeof(double));
+        if (r != CB_OK) return r;
+        for (size_t at = 0; at < rows && e == cudaSuccess; at += most) {
+            const size_t m = std::min(most, rows - at);
+            e = cudaMemcpyAsync(h->tmp, src + at * n, m * n * sizeof(double), cudaMemcpyHostToDevice, h->stream);
+            if (e == cudaSuccess)
+                e = launch_repitch(P_FP64, h->prec, h->tmp, n, (char *)dst + at * pitch * h->esz, pitch, (int)n, m,
+                                   h->stream);
+        }
+    } else if (h->prec == P_FP64) {
         e = cudaMemcpyAsync(dst, src, h->N * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     } else {
         int r = ensure_tmp(h, h->N * sizeof(double));
@@ -360,7 +397,7 @@ int upload_field(cb_handle *h, void *dst, const double *src) {
 
 /* Release the staging buffer after the set-up (FP32C uploads need N doubles). */
 void release_tmp(cb_handle *h) {
-    if (h->tmp && h->prec == P_FP32) {
+    if (h->tmp && (h->prec == P_FP32 || h->k.pitch != h->p.n_grids)) {
         cudaFreeAsync(h->tmp, h->stream);
         h->tmp = nullptr;
         h->tmp_bytes = 0;
@@ -665,10 +702,8 @@ int64_t cb_footprint_bytes(const cb_params *p) {
     std::string why;
     if (validate_params(p, why) != CB_OK) return CB_EINVAL;
     StepConst k = make_const(p);
-    size_t N = 1;
-    for (int i = 0; i < p->d; ++i) N *= (size_t)p->n_grids;
     const size_t esz = p->precision == CB_FP64 ? 8 : 4;
-    size_t b = N * esz * (4 + (p->memorysave == 0 ? 3 : 0));
+    size_t b = field_elems(k) * esz * (4 + (p->memorysave == 0 ? 3 : 0));
     b += std::max(step_blocks(k), ic_blocks(k)) * NSUM * sizeof(double) + sizeof(DevState);
     return (int64_t)b;
 }
@@ -715,7 +750,7 @@ int cb_create_from_ic(const cb_params *p, const double *phi0, const double *pi0,
     r = upload_field(h, h->phi[0], phi0);
     if (r == CB_OK) {
         if (pi0) r = upload_field(h, h->pi[0], pi0);
-        else if (cudaMemsetAsync(h->pi[0], 0, h->N * h->esz, h->stream) != cudaSuccess) r = CB_EDEVICE;
+        else if (cudaMemsetAsync(h->pi[0], 0, field_elems(h->k) * h->esz, h->stream) != cudaSuccess) r = CB_EDEVICE;
     }
     if (r != CB_OK) {
         g_create_error = h->err.empty() ? "uploading the initial condition failed" : h->err;
@@ -841,7 +876,17 @@ int cb_get_fields(cb_handle *h, double *phi, double *pi, double *ekin, double *e
         for (int f = 0; f < 5; ++f) {
             if (!dst[f]) continue;
             cudaError_t e;
-            if (h->prec == P_FP64) {
+            if (h->k.pitch != h->p.n_grids) {
+                void *to = dst[f];
+                if (h->prec == P_FP32) {
+                    tmp.resize(h->N);
+                    to = tmp.data();
+                }
+                e = download_padded(h, src[f], h->prec, to, r);
+                if (r != CB_OK) return r;
+                if (e == cudaSuccess && h->prec == P_FP32)
+                    for (size_t i = 0; i < h->N; ++i) dst[f][i] = (double)tmp[i];
+            } else if (h->prec == P_FP64) {
                 e = cudaMemcpyAsync(dst[f], src[f], h->N * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
                 if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
             } else {
@@ -865,10 +910,17 @@ int cb_get_fields_f32(cb_handle *h, float *phi, float *pi, float *ekin, float *e
     if (r != CB_OK) return r;
     const void *src[5] = {h->phi[h->cphi], h->pi[h->cpi], h->loc[0], h->loc[1], h->loc[2]};
     float *dst[5] = {phi, pi, ekin, egrad, epot};
-    if (h->prec == P_FP64 && (r = ensure_tmp(h, h->N * sizeof(float))) != CB_OK) return r;
+    const bool padded = h->k.pitch != h->p.n_grids;
+    if (!padded && h->prec == P_FP64 && (r = ensure_tmp(h, h->N * sizeof(float))) != CB_OK) return r;
     for (int f = 0; f < 5; ++f) {
         if (!dst[f]) continue;
         cudaError_t e = cudaSuccess;
+        if (padded) {
+            e = download_padded(h, src[f], P_FP32, dst[f], r);
+            if (r != CB_OK) return r;
+            if (e != cudaSuccess) return cuda_fail(h, e, "downloading a field");
+            continue;
+        }
         const void *from = src[f];
         if (h->prec == P_FP64) {
             e = launch_convert(P_FP64, P_FP32, src[f], h->tmp, h->N, h->stream);

@@ -213,7 +213,7 @@ __device__ double2 *fft_smem(double2 *a, double2 *b, const Plan &pl, int C, cons
 
 /* Last axis: C row pairs per block. Row pair p covers rows 2p, 2p+1. */
 template <typename T>
-__global__ void __launch_bounds__(FFT_T) k_fft_rows(Plan pl, const T *__restrict__ field, size_t rows, int C,
+__global__ void __launch_bounds__(FFT_T) k_fft_rows(Plan pl, const T *__restrict__ field, size_t fpitch, size_t rows, int C,
                                                    const double2 *__restrict__ tw, double2 *__restrict__ out) {
     extern __shared__ double2 sm[];
     const int n = pl.n, h = n / 2 + 1;
@@ -231,8 +231,8 @@ __global__ void __launch_bounds__(FFT_T) k_fft_rows(Plan pl, const T *__restrict
                 int c, i;
                 divmod(idx, n, pl.logn, c, i);
                 const size_t ra = 2 * (p0 + c), rb = ra + 1;
-                if (ra < rows) xa[u] = __ldg(&field[ra * n + i]);
-                if (rb < rows) xb[u] = __ldg(&field[rb * n + i]);
+                if (ra < rows) xa[u] = __ldg(&field[ra * fpitch + i]);
+                if (rb < rows) xb[u] = __ldg(&field[rb * fpitch + i]);
             }
         }
 #pragma unroll
@@ -927,8 +927,8 @@ cudaError_t fft_r2c_reg(FftState *f, int prec, const void *field, cudaStream_t s
     }
 }
 
-/* r2c of `field` (n^d values of the given precision) into f->half. */
-cudaError_t fft_r2c(FftState *f, int prec, const void *field, cudaStream_t s) {
+/* r2c of `field` (rows of n values, fpitch apart, of the given precision) into f->half. */
+cudaError_t fft_r2c(FftState *f, int prec, const void *field, int fpitch, cudaStream_t s) {
     if (f->reg) return fft_r2c_reg(f, prec, field, s);
     const int n = f->n, d = f->d;
     Plan pl = plan_of(*f);
@@ -942,11 +942,11 @@ cudaError_t fft_r2c(FftState *f, int prec, const void *field, cudaStream_t s) {
     if (prec == P_FP64) {
         e = cudaFuncSetAttribute(k_fft_rows<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        k_fft_rows<double><<<grid_rows, FFT_T, sm, s>>>(pl, (const double *)field, rows, C, f->tw, f->half);
+        k_fft_rows<double><<<grid_rows, FFT_T, sm, s>>>(pl, (const double *)field, (size_t)fpitch, rows, C, f->tw, f->half);
     } else {
         e = cudaFuncSetAttribute(k_fft_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
-        k_fft_rows<float><<<grid_rows, FFT_T, sm, s>>>(pl, (const float *)field, rows, C, f->tw, f->half);
+        k_fft_rows<float><<<grid_rows, FFT_T, sm, s>>>(pl, (const float *)field, (size_t)fpitch, rows, C, f->tw, f->half);
     }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const int hh = n / 2 + 1;
@@ -1040,7 +1040,7 @@ extern "C" int cb_power_spectrum(cb_handle *h, double *power, double *weight, do
             const BinConst bc = bin_const(h->fft, h->p.L);
             e = fft_r2c_reg(h->fft, h->prec, h->phi[h->cphi], h->stream, &bc);
         } else {
-            e = fft_r2c(h->fft, h->prec, h->phi[h->cphi], h->stream);
+            e = fft_r2c(h->fft, h->prec, h->phi[h->cphi], h->k.pitch, h->stream);
             if (e == cudaSuccess) e = fft_bins(h->fft, h->p.L, h->stream);
         }
         std::vector<double> host(3 * (size_t)nb);
@@ -1118,7 +1118,7 @@ extern "C" int cb_dft_r2c(int d, int n, const double *in, double *out) {
         double *dev = nullptr;
         e = cudaMalloc(&dev, N * sizeof(double));
         if (e == cudaSuccess) e = cudaMemcpyAsync(dev, in, N * sizeof(double), cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = fft_r2c(f, P_FP64, dev, s);
+        if (e == cudaSuccess) e = fft_r2c(f, P_FP64, dev, n, s);
         const size_t hh = (size_t)n / 2 + 1;
         if (e == cudaSuccess)
             e = cudaMemcpy2DAsync(out, hh * sizeof(double2), f->half, (size_t)f->pitch * sizeof(double2),

@@ -45,12 +45,20 @@ Fits fits(double c, int d) {
     return f;
 }
 
+/* site s of a field of rows `pitch` apart, and its image in the row's pad */
+template <typename T>
+__device__ __forceinline__ void put_site(T *f, size_t s, int n, int pitch, T v) {
+    const size_t r = s / (size_t)n, c = s - r * (size_t)n;
+    f[r * (size_t)pitch + c] = v;
+    if (n + c < (size_t)pitch) f[r * (size_t)pitch + n + c] = v;
+}
+
 /* phi(s) = min(phi + (phi_C/2)(tanh((R - |x - x_b|)/w) + 1), phi_C) over the
  * positions in file order (bubble.cpp:102-108, 434-448); the other modes as
  * their reference routines (324-393). */
 template <typename T>
 __global__ void k_ic_profiles(int d, int n, double L, int mode, int test, double deltar, Fits f,
-                              const double *__restrict__ xyz, int npos, T *__restrict__ phi, size_t N) {
+                              const double *__restrict__ xyz, int npos, T *__restrict__ phi, int pitch, size_t N) {
     for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < N; s += (size_t)gridDim.x * blockDim.x) {
         double x[3] = {0.0, 0.0, 0.0};
         const size_t nn = (size_t)n;
@@ -90,14 +98,15 @@ __global__ void k_ic_profiles(int d, int n, double L, int mode, int test, double
                 v = fmin(v + prof(d == 2 ? a0 * a0 + a1 * a1 : a0 * a0 + a1 * a1 + a2 * a2), f.phic);
             }
         }
-        phi[s] = (T)v;
+        put_site(phi, s, n, pitch, (T)v);
     }
 }
 
 template <typename T>
-__global__ void k_scale_into(const double *__restrict__ src, double norm, T *__restrict__ dst, size_t N) {
+__global__ void k_scale_into(const double *__restrict__ src, double norm, T *__restrict__ dst, int n, int pitch,
+                             size_t N) {
     for (size_t s = blockIdx.x * (size_t)blockDim.x + threadIdx.x; s < N; s += (size_t)gridDim.x * blockDim.x)
-        dst[s] = (T)(src[s] * norm + 0.0);
+        put_site(dst, s, n, pitch, (T)(src[s] * norm + 0.0));
 }
 
 unsigned grid_for(size_t N) {
@@ -115,7 +124,7 @@ int device_initial_condition(cb_handle *h, const cb_ic_params *ic, const char *x
     const size_t N = h->N;
     void *phi = h->phi[0], *pi = h->pi[0];
     cudaStream_t s = h->stream;
-    cudaError_t e = cudaMemsetAsync(pi, 0, N * h->esz, s);
+    cudaError_t e = cudaMemsetAsync(pi, 0, field_elems(h->k) * h->esz, s);
     if (e != cudaSuccess) return cuda_fail(h, e, "initial condition");
     const Fits f = fits(c, d);
     if (d >= 2 && !ic->test && ic->mode == -3) {
@@ -133,8 +142,8 @@ int device_initial_condition(cb_handle *h, const cb_ic_params *ic, const char *x
             if (r == CB_OK) r = device_c2r(d, n, half.data(), tmp, s);
             if (r != CB_OK) { cudaFreeAsync(tmp, s); return fail(h, r, "initial condition: inverse DFT"); }
             void *dst = which == 0 ? phi : pi;
-            if (h->prec == P_FP64) k_scale_into<double><<<grid_for(N), 256, 0, s>>>(tmp, norm, (double *)dst, N);
-            else k_scale_into<float><<<grid_for(N), 256, 0, s>>>(tmp, norm, (float *)dst, N);
+            if (h->prec == P_FP64) k_scale_into<double><<<grid_for(N), 256, 0, s>>>(tmp, norm, (double *)dst, n, h->k.pitch, N);
+            else k_scale_into<float><<<grid_for(N), 256, 0, s>>>(tmp, norm, (float *)dst, n, h->k.pitch, N);
         }
         cudaFreeAsync(tmp, s);
         e = cudaStreamSynchronize(s);
@@ -164,10 +173,10 @@ int device_initial_condition(cb_handle *h, const cb_ic_params *ic, const char *x
     }
     if (h->prec == P_FP64)
         k_ic_profiles<double><<<grid_for(N), 256, 0, s>>>(d, n, L, ic->mode, ic->test, ic->deltar, f, dxyz, npos,
-                                                         (double *)phi, N);
+                                                         (double *)phi, h->k.pitch, N);
     else
         k_ic_profiles<float><<<grid_for(N), 256, 0, s>>>(d, n, L, ic->mode, ic->test, ic->deltar, f, dxyz, npos,
-                                                        (float *)phi, N);
+                                                        (float *)phi, h->k.pitch, N);
     if (dxyz) cudaFreeAsync(dxyz, s);
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(h, e, "initial condition");

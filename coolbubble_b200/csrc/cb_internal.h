@@ -68,6 +68,9 @@ struct StepConst {
     int d, n;
     int ni, nj, nk;     /* extents mapped onto (march axis, tile rows, tile columns) */
     int cz;             /* planes per block along the march axis (generic d = 3 kernel) */
+    int pitch;          /* elements from a row of the last axis to the next: n, or (d = 3 runs) n rounded
+                           up to whole 16-byte vectors. The pad holds the periodic images of the row's
+                           first sites: every kernel that writes phi or pi keeps them equal */
     double dt;
     double c2, c3, c4;  /* V'(f) = c2 f - c3 f^2 + c4 f^3, coefficients as bubble.cpp:76 forms them */
     double v2, v3, v4, dv; /* V(f) = v2 f^2 - v3 f^3 + v4 f^4 + DeltaV (bubble.cpp:71) */
@@ -164,6 +167,21 @@ size_t ic_blocks(const StepConst &k);
 cudaError_t launch_flush_drift(int prec, const StepConst &k, const void *phi, const void *pi, void *phi_out,
                                DevState *st, cudaStream_t s);
 cudaError_t launch_convert(int from_prec, int to_prec, const void *src, void *dst, size_t n, cudaStream_t s);
+/* `rows` rows of n elements between a field's rows (k.pitch apart) and dense
+ * ones, converted on the way; a padded destination gets its images */
+cudaError_t launch_repitch(int from_prec, int to_prec, const void *src, size_t src_pitch, void *dst, size_t dst_pitch,
+                           int n, size_t rows, cudaStream_t s);
+/* elements of a field's buffer, pads included */
+inline size_t field_elems(const StepConst &k) {
+    size_t e = (size_t)k.pitch;
+    for (int i = 1; i < k.d; ++i) e *= (size_t)k.n;
+    return e;
+}
+/* a d = 3 run's row pitch: whole 16-byte vectors where the staged kernels apply */
+inline int run_pitch(int d, int n, int prec) {
+    const int W = prec == 0 ? 2 : 4;
+    return d == 3 && n >= 64 ? (n + W - 1) / W * W : n;
+}
 
 }  // namespace cb
 

@@ -19,7 +19,7 @@ namespace cb {
 namespace {
 
 template <typename T>
-__global__ void k_gather_line(int d, int n, int i0, int i1, int i2, int count, const T *__restrict__ phi,
+__global__ void k_gather_line(int d, int n, int pitch, int i0, int i1, int i2, int count, const T *__restrict__ phi,
                               const T *__restrict__ pi, bool pending, T dt, const DevState *st,
                               double *__restrict__ out) {
     using A = Ar<T>;
@@ -29,7 +29,7 @@ __global__ void k_gather_line(int d, int n, int i0, int i1, int i2, int count, c
     size_t s;
     if (d == 1) s = (size_t)i;
     else if (d == 2) s = (size_t)i * n + i1;
-    else s = ((size_t)i * n + i1) * n + i2;
+    else s = ((size_t)i * n + i1) * pitch + i2;
     T v = phi[s];
     if (pending) v = A::add(v, A::mul(A::mul(dt, pi[s]), (T)st->drift_p));   /* bubble.cpp:867-870 */
     out[m] = (double)v;
@@ -53,11 +53,11 @@ extern "C" int cb_get_line(cb_handle *h, int i0, int i1, int i2, int count, doub
     double *dev = static_cast<double *>(h->tmp);
     const unsigned blocks = (unsigned)((count + 127) / 128);
     if (h->prec == P_FP64)
-        k_gather_line<double><<<blocks, 128, 0, h->stream>>>(d, n, i0, i1, i2, count, (const double *)h->phi[h->cphi],
+        k_gather_line<double><<<blocks, 128, 0, h->stream>>>(d, n, h->k.pitch, i0, i1, i2, count, (const double *)h->phi[h->cphi],
                                                              (const double *)h->pi[h->cpi], h->pending, h->k.dt,
                                                              h->st, dev);
     else
-        k_gather_line<float><<<blocks, 128, 0, h->stream>>>(d, n, i0, i1, i2, count, (const float *)h->phi[h->cphi],
+        k_gather_line<float><<<blocks, 128, 0, h->stream>>>(d, n, h->k.pitch, i0, i1, i2, count, (const float *)h->phi[h->cphi],
                                                             (const float *)h->pi[h->cpi], h->pending, h->k.dtf,
                                                             h->st, dev);
     cudaError_t e = cudaGetLastError();

@@ -76,6 +76,7 @@ extern "C" int cb_step_static_noalloc(const cb_params *p, const void *phi_in, co
         return fail(nullptr, CB_EINVAL, "cb_step_static_noalloc: output buffers must differ from the inputs");
     StepConst k = make_const(p);
     k.want_local = 0;
+    k.pitch = k.n;   /* the caller's rows are dense */
     const size_t blocks = step_blocks(k);
     if (blocks > NOALLOC_MAX_BLOCKS) {
         char b[200];

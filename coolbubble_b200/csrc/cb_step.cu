@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(TX *TY) k_step(StepConst k, const T *__restric
     const int kk = blockIdx.x * TX + tx;
     const int jj = blockIdx.y * TY + ty;
     const bool active = kk < nk && jj < nj;
-    const size_t sj = (size_t)nk, si = (size_t)nj * nk;
+    const size_t sj = (size_t)k.pitch, si = (size_t)nj * k.pitch;
     const size_t col = (size_t)(jj % nj) * sj + (size_t)(kk % nk);
     const int i0 = (D == 3) ? blockIdx.z * k.cz : 0;
     const int i1 = (D == 3) ? min(i0 + k.cz, ni) : 1;
@@ -131,8 +131,13 @@ __global__ void __launch_bounds__(TX *TY) k_step(StepConst k, const T *__restric
             const T pinew = A::add(pic, A::mul(dt, force));
             const size_t o = base + col;
             T eg_site = (T)0;
+            const T phinew = DF ? cur : A::add(cur, A::mul(dt, pinew));
             pi_out[o] = pinew;
-            phi_out[o] = DF ? cur : A::add(cur, A::mul(dt, pinew));
+            phi_out[o] = phinew;
+            if (D == 3 && kk < k.pitch - nk) {   /* the image in the row's pad */
+                pi_out[o + nk] = pinew;
+                phi_out[o + nk] = phinew;
+            }
             if (SUMS == SUM_FULL || (SUMS == SUM_FRIEDMANN && k.alpha == 1)) {
                 /* forward gradients in the reference's naming (bubble.cpp:788-801) */
                 T gx, gy = (T)0, gz = (T)0;
@@ -195,18 +200,27 @@ __global__ void __launch_bounds__(TX *TY) k_step(StepConst k, const T *__restric
 
 /* ---- set-up kernels (once per run; plain global loads, through L1/L2) --- */
 
+/* site s of the lattice as an element of a field (rows k.pitch apart) */
+__device__ __forceinline__ size_t elem_of(const StepConst &k, size_t s) {
+    return k.pitch == k.n ? s : s + s / (size_t)k.n * (size_t)(k.pitch - k.n);
+}
+
+/* the element of site s's neighbour along an axis, for lattices of 2^32 sites and more */
 __device__ __forceinline__ size_t nb_index(const StepConst &k, size_t s, int axis, int dir) {
-    size_t stride = 1;
-    for (int a = axis + 1; a < k.d; ++a) stride *= (size_t)k.n;
+    size_t stride = 1, estride = 1;
+    for (int a = axis + 1; a < k.d; ++a) {
+        stride *= (size_t)k.n;
+        estride *= (size_t)(a == k.d - 1 ? k.pitch : k.n);
+    }
     const size_t coord = (s / stride) % (size_t)k.n;
     const size_t moved = (coord + (size_t)k.n + (size_t)(dir > 0 ? 1 : k.n - 1)) % (size_t)k.n;
-    return s - coord * stride + moved * stride;
+    return elem_of(k, s) - coord * estride + moved * estride;
 }
 
 template <typename T>
 __device__ __forceinline__ T load_as(const void *p, size_t i) { return static_cast<const T *>(p)[i]; }
 
-/* Periodic neighbours of site s for lattices of fewer than 2^32 sites: the
+/* Element and periodic neighbours of a site for fields of fewer than 2^32 elements: the
  * coordinates are taken once per site (32-bit divisions), each neighbour is
  * then an add or a wrap along its axis (axis 0 has the largest stride, as
  * gridfuncs.cpp:25-51). */
@@ -214,14 +228,16 @@ struct Site32 {
     unsigned s, n;
     unsigned c[3], stride[3];
     int d;
-    __device__ __forceinline__ Site32(const StepConst &k, unsigned site) : s(site), n((unsigned)k.n), d(k.d) {
+    __device__ __forceinline__ Site32(const StepConst &k, unsigned site) : n((unsigned)k.n), d(k.d) {
         unsigned rest = site, st = 1;
+        s = 0;
         for (int ax = 2; ax >= 0; --ax) {
             if (ax < d) {
                 c[ax] = rest % n;
                 rest /= n;
                 stride[ax] = st;
-                st *= n;
+                s += c[ax] * st;
+                st *= ax == d - 1 ? (unsigned)k.pitch : n;
             } else {
                 c[ax] = 0;
                 stride[ax] = 0;
@@ -246,9 +262,10 @@ __global__ void __launch_bounds__(NT) k_ic_energies(StepConst k, size_t N, const
 #pragma unroll
     for (int s = 0; s < NSUM; ++s) v[s] = 0.0;
     const double dx = k.dx;
-    const bool small = N < (1ull << 32);
+    const bool small = N / (size_t)k.n * (size_t)k.pitch < (1ull << 32);
     for (size_t s = blockIdx.x * (size_t)NT + threadIdx.x; s < N; s += (size_t)gridDim.x * NT) {
-        const double f = (double)phi[s];
+        const size_t e = elem_of(k, s);
+        const double f = (double)phi[e];
         double g2 = 0.0;
         if (small) {
             const Site32 q(k, (unsigned)s);
@@ -266,12 +283,12 @@ __global__ void __launch_bounds__(NT) k_ic_energies(StepConst k, size_t N, const
         }
         const double eg = __dmul_rn(0.5, g2);
         const double ep = Vpot<double>(k, f);
-        const double pv = (double)pi[s];
+        const double pv = (double)pi[e];
         const double ek = __dmul_rn(__dmul_rn(0.5, pv), pv);
         if (k.want_local) {
-            loc_ek[s] = (T)ek;
-            loc_eg[s] = (T)eg;
-            loc_ep[s] = (T)ep;
+            loc_ek[e] = (T)ek;
+            loc_eg[e] = (T)eg;
+            loc_ep[e] = (T)ep;
         }
         v[S_PHI] = __dadd_rn(v[S_PHI], f);
         v[S_V] = __dadd_rn(v[S_V], pv);
@@ -330,9 +347,10 @@ __global__ void __launch_bounds__(NT) k_ic_backkick(StepConst k, size_t N, const
     const double w = __dmul_rn(0.5, pow(a_mhalf, (double)(-2 * k.d)));
     const T fl = (T)pow(st->a, (double)(k.d - 2 + k.alpha)), fv = (T)pow(st->a, (double)(k.d + k.alpha));
     const T hdt = (T)__dmul_rn(0.5, k.dt);
-    const bool small = N < (1ull << 32);
+    const bool small = N / (size_t)k.n * (size_t)k.pitch < (1ull << 32);
     for (size_t s = blockIdx.x * (size_t)NT + threadIdx.x; s < N; s += (size_t)gridDim.x * NT) {
-        const T f = phi[s];
+        const size_t e = elem_of(k, s);
+        const T f = phi[e];
         const T two = A::add(f, f);
         T lap = (T)0;
         if (small) {
@@ -352,8 +370,9 @@ __global__ void __launch_bounds__(NT) k_ic_backkick(StepConst k, size_t N, const
         const T flap = A::mul(fl, lap);
         const T force = A::sub(k.dx2_pow2 ? A::mul(flap, kc<T>(k.inv_dx2, k.inv_dx2f)) : A::div(flap, kc<T>(k.dx2, k.dx2f)),
                                A::mul(fv, dV<T>(k, f)));
-        const T pv = A::sub(pi[s], A::mul(hdt, force));
-        pi[s] = pv;
+        const T pv = A::sub(pi[e], A::mul(hdt, force));
+        pi[e] = pv;
+        if (k.pitch != k.n && s % (size_t)k.n < (size_t)(k.pitch - k.n)) pi[e + k.n] = pv;   /* its image */
         const double pd = (double)pv;
         v[S_EK] = __dadd_rn(v[S_EK], __dmul_rn(__dmul_rn(w, pd), pd));
     }
@@ -377,6 +396,17 @@ template <typename S, typename D>
 __global__ void k_convert(const S *__restrict__ src, D *__restrict__ dst, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         dst[i] = (D)src[i];
+}
+
+template <typename S, typename D>
+__global__ void k_repitch(const S *__restrict__ src, size_t src_pitch, D *__restrict__ dst, size_t dst_pitch, int n,
+                          size_t count) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
+        const size_t r = i / (size_t)n, c = i - r * (size_t)n;
+        const D v = (D)src[r * src_pitch + c];
+        dst[r * dst_pitch + c] = v;
+        if (n + c < dst_pitch) dst[r * dst_pitch + n + c] = v;
+    }
 }
 
 constexpr int TX3 = 32, TY3 = 8;   /* d = 2, 3 tile: 32 columns x 8 rows */
@@ -458,7 +488,10 @@ cudaError_t launch_step(int prec, const StepConst &k, bool drift_first, int sums
     unsigned g3;
     if (step2_applies(k, prec, drift_first))
         return launch_step2(prec, k, sums, phi_in, pi_in, phi_out, pi_out, loc_ek, loc_eg, loc_ep, st, partials, s);
-    if (!k.force_generic && step3_geometry(k, prec, tj, ns, sm, g3))
+    /* padded rows in float: the reporting step stays with the generic kernel, whose
+     * sums are compensated per site (the staged kernel's averages are plain pair sums) */
+    const bool plain_sums = k.pitch != k.n && prec == P_FP32 && sums == SUM_FULL;
+    if (!k.force_generic && !plain_sums && step3_geometry(k, prec, tj, ns, sm, g3))
         return launch_step3(prec, k, drift_first, sums, phi_in, pi_in, phi_out, pi_out, loc_ek, loc_eg, loc_ep, st,
                             partials, s);
     if (prec == P_FP64)
@@ -495,7 +528,7 @@ cudaError_t launch_ic_backkick(int prec, const StepConst &k, const void *phi, vo
 
 cudaError_t launch_flush_drift(int prec, const StepConst &k, const void *phi, const void *pi, void *phi_out,
                                DevState *st, cudaStream_t s) {
-    const size_t N = sites(k);
+    const size_t N = field_elems(k);   /* the images in the pads too */
     if (prec == P_FP64)
         k_flush_drift<double, NT_IC><<<ic_grid(N), NT_IC, 0, s>>>(N, k.dt, (const double *)phi, (const double *)pi,
                                                                   (double *)phi_out, st);
@@ -511,6 +544,25 @@ cudaError_t launch_convert(int from, int to, const void *src, void *dst, size_t 
     if (from == P_FP64 && to == P_FP32) k_convert<double, float><<<g, NT_IC, 0, s>>>((const double *)src, (float *)dst, n);
     else if (from == P_FP32 && to == P_FP64) k_convert<float, double><<<g, NT_IC, 0, s>>>((const float *)src, (double *)dst, n);
     else return cudaErrorInvalidValue;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_repitch(int from, int to, const void *src, size_t src_pitch, void *dst, size_t dst_pitch, int n,
+                           size_t rows, cudaStream_t s) {
+    const size_t count = rows * (size_t)n;
+    const unsigned g = ic_grid(count);
+    auto go = [&](auto sv, auto dv) {
+        using S = decltype(sv);
+        using D = decltype(dv);
+        k_repitch<S, D><<<g, NT_IC, 0, s>>>((const S *)src, src_pitch, (D *)dst, dst_pitch, n, count);
+    };
+    if (from == P_FP64) {
+        if (to == P_FP64) go(0.0, 0.0);
+        else go(0.0, 0.f);
+    } else {
+        if (to == P_FP64) go(0.f, 0.0);
+        else go(0.f, 0.f);
+    }
     return cudaGetLastError();
 }
 

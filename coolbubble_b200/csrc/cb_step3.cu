@@ -17,6 +17,11 @@
  *  - The grid is one block per resident slot (2 per SM); blocks take items
  *    from a device-wide queue. Each item's box sums go to its own row of
  *    partial sums, so the totals do not depend on which block took it.
+ *  - Rows are whole 16-byte vectors: n a multiple of one, or rows padded to it
+ *    (RAG) whose pad repeats the row's first sites; the images advance with the
+ *    same vector operations as the sites and take no part in the sums. 250^3 in
+ *    float, which the generic kernel took site by site at 88 us per step, runs at
+ *    48 here and 29.7 in two-step passes (256^3: 50 and 28).
  *  - Each thread updates 16-byte vectors (4 floats / 2 doubles) and stores
  *    phi and pi with 128-bit coalesced writes.
  *  - Drift-first (expanding background): the pending drift of the previous
@@ -152,7 +157,7 @@ struct AccF2 {
  * halo rows of pi to drift the halo of phi). */
 template <typename T, bool DF>
 struct StageGeom {
-    int n, tj;
+    int n, tj;   /* elements of a row, rows of a tile */
     __device__ __forceinline__ size_t phi_elems() const { return (size_t)(tj + 2) * n; }
     __device__ __forceinline__ size_t pi_rows() const { return (size_t)(tj + (DF ? 2 : 0)); }
     __device__ __forceinline__ size_t elems() const { return phi_elems() + pi_rows() * n; }
@@ -166,7 +171,7 @@ struct StageGeom {
  * the same fixed order and runs the Friedmann update itself (block 0 also on
  * the global state), while its copies of the next step's first planes are in
  * flight. Item rows alternate between two halves of partials by step. */
-template <typename T, bool DF, int SUMS, bool MS = false>
+template <typename T, bool DF, int SUMS, bool RAG = false, bool MS = false>
 __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstage, int parts, int nsteps,
                                                 const T *phi_in, const T *pi_in, T *phi_out, T *pi_out,
                                                 T *__restrict__ loc_ek, T *__restrict__ loc_eg,
@@ -179,8 +184,8 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
     constexpr bool UNI = DF || SUMS != SUM_NONE;       /* consumers leave together */
     constexpr int NS = SUMS == SUM_FULL ? NSUM : 3;    /* sums carried (S_EK, S_EP, S_EG first) */
     extern __shared__ __align__(128) unsigned char smraw[];
-    const int n = k.n;
-    const StageGeom<T, DF> g{n, tj};
+    const int n = k.n, np = RAG ? k.pitch : n;   /* sites and elements of a row */
+    const StageGeom<T, DF> g{np, tj};
     const size_t stage_elems = g.elems();
     uint64_t *full = reinterpret_cast<uint64_t *>(smraw);
     uint64_t *empty = full + 8;
@@ -198,7 +203,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
     T *const fphi[2] = {const_cast<T *>(phi_in), phi_out};
     T *const fpi[2] = {const_cast<T *>(pi_in), pi_out};
 
-    const int ntiles = n / tj;
+    const int ntiles = RAG ? (n + tj - 1) / tj : n / tj;
     /* Work items: (plane part, tile), part-major with tiles fastest; part c
      * covers planes [c n / parts, (c + 1) n / parts). Blocks take items from a
      * device-wide queue (an atomic counter in the device state), so the items
@@ -209,9 +214,10 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
      * producer hands each item to the consumers through a small shared queue
      * guarded by its own mbarriers. */
     const int items = ntiles * parts;
-    const size_t row_bytes = (size_t)n * sizeof(T);
-    const size_t plane = (size_t)n * n;
-    const uint32_t tx_bytes = (uint32_t)(((size_t)(tj + 2) + g.pi_rows()) * row_bytes);
+    const size_t row_bytes = (size_t)np * sizeof(T);
+    const size_t plane = (size_t)n * np;
+    /* rows of the tile from row j0 (RAG: the last one may be short) */
+    auto rows_at = [&](int j0) { return RAG ? min(tj, n - j0) : tj; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto item_of = [&](int it, int &t, int &p0, int &p1) {
         const int c = it / ntiles;
@@ -248,22 +254,23 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
          *      warps released the plane it held ---- */
         auto issue = [&](int s, int pl, int j0, int sb) {
             const int pw = pl < 0 ? pl + n : (pl >= n ? pl - n : pl);
-            const int jm = (j0 - 1 + n) % n, jp = (j0 + tj) % n;
+            const int tr = rows_at(j0);
+            const int jm = (j0 - 1 + n) % n, jp = (j0 + tr) % n;
             T *dst = ring + (size_t)s * stage_elems;
             const T *src_phi = fphi[sb] + (size_t)pw * plane;
             const T *src_pi = fpi[sb] + (size_t)pw * plane;
             fence_proxy_async();
-            mbar_arrive_expect_tx(&full[s], tx_bytes);
-            bulk_g2s(dst + n, src_phi + (size_t)j0 * n, (uint32_t)(tj * row_bytes), &full[s]);
-            bulk_g2s(dst, src_phi + (size_t)jm * n, (uint32_t)row_bytes, &full[s]);
-            bulk_g2s(dst + (size_t)(tj + 1) * n, src_phi + (size_t)jp * n, (uint32_t)row_bytes, &full[s]);
+            mbar_arrive_expect_tx(&full[s], (uint32_t)((2 * tr + (DF ? 4 : 2)) * row_bytes));
+            bulk_g2s(dst + np, src_phi + (size_t)j0 * np, (uint32_t)(tr * row_bytes), &full[s]);
+            bulk_g2s(dst, src_phi + (size_t)jm * np, (uint32_t)row_bytes, &full[s]);
+            bulk_g2s(dst + (size_t)(tr + 1) * np, src_phi + (size_t)jp * np, (uint32_t)row_bytes, &full[s]);
             T *dpi = dst + g.phi_elems();
             if (DF) {
-                bulk_g2s(dpi + n, src_pi + (size_t)j0 * n, (uint32_t)(tj * row_bytes), &full[s]);
-                bulk_g2s(dpi, src_pi + (size_t)jm * n, (uint32_t)row_bytes, &full[s]);
-                bulk_g2s(dpi + (size_t)(tj + 1) * n, src_pi + (size_t)jp * n, (uint32_t)row_bytes, &full[s]);
+                bulk_g2s(dpi + np, src_pi + (size_t)j0 * np, (uint32_t)(tr * row_bytes), &full[s]);
+                bulk_g2s(dpi, src_pi + (size_t)jm * np, (uint32_t)row_bytes, &full[s]);
+                bulk_g2s(dpi + (size_t)(tr + 1) * np, src_pi + (size_t)jp * np, (uint32_t)row_bytes, &full[s]);
             } else {
-                bulk_g2s(dpi, src_pi + (size_t)j0 * n, (uint32_t)(tj * row_bytes), &full[s]);
+                bulk_g2s(dpi, src_pi + (size_t)j0 * np, (uint32_t)(tr * row_bytes), &full[s]);
             }
         };
         /* stage reuse: position q goes where position q - nstage was, once
@@ -349,8 +356,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
             const bool dx2_pow2 = std::is_same<T, float>::value || k.dx2_pow2 != 0;
             const T half = (T)0.5;
             auto grad = [&](T dphi) -> T { return adx_pow2 ? A::mul(dphi, inv_adx) : A::div(dphi, adx); };
-            const int nvec_row = n / W;
-            const int nvec = tj * nvec_row;
+            const int nvec_row = np / W;
             const int row_step = NC / nvec_row, vec_step = NC % nvec_row;
             constexpr bool want_eg = SUMS == SUM_FULL || SUMS == SUM_FRIEDMANN_EG;
             /* float steps run in packed f32x2 pairs, with or without sums */
@@ -377,8 +383,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
              * Each thread drifts its share of a plane two planes ahead of the one it
              * computes and arrives on the plane's drift mbarrier, so the consumer
              * warps only wait for each other where a plane is first read. */
-            const int nv_drift = (tj + 2) * n / W;
-            auto drift_share = [&](const Cursor &c) {
+            auto drift_share = [&](const Cursor &c, int nv_drift) {
                 T *S = ring + c.s * stage_n;
                 const T *Pi = S + pi_off;
                 for (int v = threadIdx.x; v < nv_drift; v += NC) {
@@ -431,7 +436,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                 }
                 int t, p0, p1;
                 item_of(it, t, p0, p1);
-                const int j0 = t * tj;
+                const int j0 = t * tj, nvec = rows_at(j0) * nvec_row, nv_drift = nvec + 2 * nvec_row;
                 if (SUMS != SUM_NONE) {
     #pragma unroll
                     for (int s = 0; s < NSUM; ++s) {
@@ -453,9 +458,9 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                      * planes two ahead of the one computed */
                     bad = !(acquire(cm) && acquire(c0) && acquire(cp));
                     if (!bad) {
-                        drift_share(cm);
-                        drift_share(c0);
-                        drift_share(cp);
+                        drift_share(cm, nv_drift);
+                        drift_share(c0, nv_drift);
+                        drift_share(cp, nv_drift);
                         bad = !(drifted_wait(cm) && drifted_wait(c0));
                     }
                 } else {
@@ -473,8 +478,8 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                     const T *Sm = ring + cm.s * stage_n;
                     const T *S0 = ring + c0.s * stage_n;
                     const T *Sp = ring + cp.s * stage_n;
-                    const T *P0 = S0 + pi_off + (DF ? n : 0);
-                    const size_t gbase = ((size_t)i * n + j0) * n;
+                    const T *P0 = S0 + pi_off + (DF ? np : 0);
+                    const size_t gbase = ((size_t)i * n + j0) * np;
                     T *const phi_o = fphi[MS ? (sp + 1) & 1 : 1] + gbase;
                     T *const pi_o = fpi[MS ? (sp + 1) & 1 : 1] + gbase;
                     int r = r_first, kv = kv_first;
@@ -484,17 +489,20 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                             ++r;
                         }
                         const int kk = kv * W;
-                        const int c_off = (r + 1) * n + kk;
+                        const int c_off = (r + 1) * np + kk;
                         const VT c = *reinterpret_cast<const VT *>(S0 + c_off);
-                        const VT um = *reinterpret_cast<const VT *>(S0 + c_off - n);
-                        const VT up = *reinterpret_cast<const VT *>(S0 + c_off + n);
+                        const VT um = *reinterpret_cast<const VT *>(S0 + c_off - np);
+                        const VT up = *reinterpret_cast<const VT *>(S0 + c_off + np);
                         const VT im = *reinterpret_cast<const VT *>(Sm + c_off);
                         const VT ip = *reinterpret_cast<const VT *>(Sp + c_off);
-                        const VT pv = *reinterpret_cast<const VT *>(P0 + r * n + kk);
-                        const int lo = (r + 1) * n + (kk == 0 ? n - 1 : kk - 1);
-                        const int ro = (r + 1) * n + (kk + W == n ? 0 : kk + W);
+                        const VT pv = *reinterpret_cast<const VT *>(P0 + r * np + kk);
+                        const int lo = (r + 1) * np + (kk == 0 ? n - 1 : kk - 1);
+                        const int ro = (r + 1) * np + (kk + W >= n ? kk + W - n : kk + W);
                         const T left = S0[lo];
                         const T right = S0[ro];
+                        /* RAG: the row's last vector holds `sites` sites, then images of the
+                         * row's first ones (which advance as those do) */
+                        const int sites = RAG ? min(W, n - kk) : W;
                         VT phi_new, pi_new, vek{}, veg{}, vep{};
                         if constexpr (PACKED) {
                         /* float: the four sites as two packed pairs (f32x2 arithmetic, one
@@ -556,6 +564,14 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                         pi_new = make_float4(f2_lo(pi01), f2_hi(pi01), f2_lo(pi23), f2_hi(pi23));
                         if constexpr (SUMS != SUM_NONE) {
                             constexpr int NA = SUMS == SUM_FULL ? NSUM : (want_eg ? 3 : 2);
+                            if (RAG && sites < W) {
+                                /* no sums of the images */
+#pragma unroll
+                                for (int q = 0; q < NA; ++q) {
+                                    v01[q] = f2_pack(f2_lo(v01[q]), sites > 1 ? f2_hi(v01[q]) : 0.f);
+                                    v23[q] = f2_pack(sites > 2 ? f2_lo(v23[q]) : 0.f, 0.f);
+                                }
+                            }
     #pragma unroll
                             for (int q = 0; q < NA; ++q) {
                                 /* the energies (and the previous half step's kinetic sum, which
@@ -607,7 +623,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                             const T pn = A::add(pic, A::mul(dt, force));
                             Vec<T>::set(pi_new, s, pn);
                             Vec<T>::set(phi_new, s, DF ? cur : A::add(cur, A::mul(dt, pn)));
-                            if (SUMS != SUM_NONE) {
+                            if (SUMS != SUM_NONE && (!RAG || s < sites)) {
                                 T eg = (T)0;
                                 if constexpr (want_eg) {
                                     /* forward gradients: x <- axis 1, y <- axis 0, z <- axis 2 (bubble.cpp:794-801) */
@@ -652,7 +668,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                             }
                         }
                         }
-                        const int o = r * n + kk;
+                        const int o = r * np + kk;
                         *reinterpret_cast<VT *>(pi_o + o) = pi_new;
                         *reinterpret_cast<VT *>(phi_o + o) = phi_new;
                         if (SUMS == SUM_FULL && k.want_local) {
@@ -676,7 +692,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj, int nstag
                             bad = true;
                             break;
                         }
-                        drift_share(cp);
+                        drift_share(cp, nv_drift);
                     }
                 }
                 if (!UNI && bad) {
@@ -810,7 +826,8 @@ int sm_count() {
     return v;
 }
 
-/* The tiled path covers d = 3 with n a multiple of the vector width, n >= 64,
+/* The tiled path covers d = 3 with rows of whole vectors (n a multiple of the
+ * vector width, or rows padded to one), n >= 64,
  * where a ring of four stages fits in 220 KB; returns false for other shapes
  * (the generic kernel runs).
  * Geometry: TJ rows per tile (TJ * n about 2048 sites in float, 1024 in
@@ -823,20 +840,23 @@ int sm_count() {
 bool step3_geometry_parts(const StepConst &k, int prec, int &tj, int &nstage, size_t &smem, unsigned &grid,
                           int &parts, bool whole_rounds = false) {
     if (k.d != 3) return false;
-    const int n = k.n;
+    const int n = k.n, np = k.pitch;
     const int esz = prec == P_FP64 ? 8 : 4;
     const int W = 16 / esz;
-    if (n % W != 0 || n < 64) return false;
+    if (np % W != 0 || n < 64) return false;
+    const bool rag = np != n;
     int tile_sites = prec == P_FP64 ? 1024 : 2048;
     const char *tenv = std::getenv("CB_STEP3_TILE");
     const bool tile_given = tenv && std::atoi(tenv) >= 64;
     if (tile_given) tile_sites = std::atoi(tenv);
     const bool df = k.expanding != 0;
-    auto stage_of = [&](int t) { return ((size_t)(t + 2) + (size_t)(t + (df ? 2 : 0))) * n * esz; };
+    auto stage_of = [&](int t) { return ((size_t)(t + 2) + (size_t)(t + (df ? 2 : 0))) * np * esz; };
     auto rows_for = [&](int sites, size_t cap) {
         int best = 0;
         for (int t = 1; t <= n && (long long)t * n <= sites; ++t)
-            if (n % t == 0 && HDR + 4 * stage_of(t) <= cap) best = t;
+            if ((rag || n % t == 0) && HDR + 4 * stage_of(t) <= cap) best = t;
+        /* ragged rows: tiles of nearly equal height, the last one shorter */
+        if (rag && best) best = (n + (n + best - 1) / best - 1) / ((n + best - 1) / best);
         return best;
     };
     /* two blocks per SM (with their static shared memory) while four stages of
@@ -857,7 +877,7 @@ bool step3_geometry_parts(const StepConst &k, int prec, int &tj, int &nstage, si
     if (nstage > 8) nstage = 8;
     if (nstage < 4) return false;
     smem = HDR + nstage * stage;
-    const long long ntiles = n / tj;
+    const long long ntiles = (n + tj - 1) / tj;
     const long long slots = (long long)per_sm * sm_count();
     /* time in units of one plane of one tile. An item costs its planes plus a
      * fixed part -- about one plane for a static background, 2.5 with
@@ -901,7 +921,7 @@ size_t step3_partial_rows(const StepConst &k, int prec) {
     unsigned grid;
     if (!step3_geometry_parts(k, prec, tj, nstage, smem, grid, parts)) return 0;
     if (!step3_geometry_parts(k, prec, tj, nstage, smem, grid, parts_full, true)) return 0;
-    const size_t rows = (size_t)(k.n / tj) * (size_t)std::max(parts, parts_full);
+    const size_t rows = (size_t)((k.n + tj - 1) / tj) * (size_t)std::max(parts, parts_full);
     return k.expanding ? 2 * rows : rows;
 }
 
@@ -915,7 +935,7 @@ cudaError_t launch_step3(int prec, const StepConst &k, bool df, int sums, const 
         return cudaErrorInvalidValue;
 #define CB_LAUNCH3(T, DFv, SU)                                                                                     \
     do {                                                                                                           \
-        auto fn = k_step3<T, DFv, SU>;                                                                             \
+        auto fn = k.pitch != k.n ? k_step3<T, DFv, SU, true> : k_step3<T, DFv, SU>;                                                                           \
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
         if (e != cudaSuccess) return e;                                                                            \
         e = launch_pdl(fn, dim3(grid), dim3(NT3), smem, s, k, tj, nstage, parts, 1, (const T *)phi_in,             \
@@ -957,8 +977,10 @@ cudaError_t launch_step3_ms_t(int prec, const StepConst &k, int nsteps, void *ph
      * saves (256^3: 0.0540 -> 0.0524 ms per step, 128^3: 0.0142 -> 0.0125);
      * with several rounds per step one launch per step measured faster
      * (384^3: 0.165 against 0.179 ms, 512^3: 0.393 against 0.404) */
-    if ((long long)(k.n / tj) * parts > (long long)grid) return cudaErrorNotSupported;
-    auto fn = k.alpha == 1 ? k_step3<T, true, SUM_FRIEDMANN_EG, true> : k_step3<T, true, SUM_FRIEDMANN, true>;
+    if ((long long)((k.n + tj - 1) / tj) * parts > (long long)grid) return cudaErrorNotSupported;
+    const bool rag = k.pitch != k.n;
+    auto fn = k.alpha == 1 ? (rag ? k_step3<T, true, SUM_FRIEDMANN_EG, true, true> : k_step3<T, true, SUM_FRIEDMANN_EG, false, true>)
+                           : (rag ? k_step3<T, true, SUM_FRIEDMANN, true, true> : k_step3<T, true, SUM_FRIEDMANN, false, true>);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

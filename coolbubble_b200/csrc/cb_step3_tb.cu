@@ -5,8 +5,7 @@
  * reported ones needs a global sum). One launch reads phi_n, pi_{n-1/2} and
  * writes phi_{n+2}, pi_{n+3/2}: half the DRAM bytes per step.
  *
- *  - Float and double; n any multiple of the 16-byte vector with rows of a warp
- *    or more. Tiles of TJ full rows of axis 1 (axis-2 neighbours wrap in shared
+ *  - Float and double; rows of a warp or more, padded to whole 16-byte vectors. Tiles of TJ full rows of axis 1 (axis-2 neighbours wrap in shared
  *    memory; the last tile may hang over the lattice's end and repeat its first
  *    rows); work items (plane part, tile) taken from a device-wide queue,
  *    part-major with tiles fastest (the items in flight share their halo rows
@@ -278,20 +277,20 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     __shared__ int abort_flag;
     __shared__ int item_q[TB_IQ];
 
-    const int n = k.n;
+    const int n = k.n, np = WHOLE ? n : k.pitch;   /* sites and elements of a row */
     const int R0 = tj + 4;                 /* input phi rows: j0 - 2 .. j0 + tj + 1 */
     const int R0p = tj + 2;                /* input pi rows: j0 - 1 .. j0 + tj */
     const int R1 = tj + 2;                 /* level-1 phi rows: j0 - 1 .. j0 + tj */
-    const int stage_n = (R0 + R0p) * n;    /* elements per input stage */
-    const int slot_n = R1 * n;             /* elements per level-1 slot */
+    const int stage_n = (R0 + R0p) * np;    /* elements per input stage */
+    const int slot_n = R1 * np;             /* elements per level-1 slot */
     uint64_t *full = reinterpret_cast<uint64_t *>(smraw);
     T *ring = reinterpret_cast<T *>(smraw + TB_HDR);
     T *l1 = ring + (size_t)nstage * stage_n;
 
     const int ntiles = (n + tj - 1) / tj;
     const int items = ntiles * parts;
-    const size_t row_bytes = (size_t)n * sizeof(T);
-    const size_t plane = (size_t)n * n;
+    const size_t row_bytes = (size_t)np * sizeof(T);
+    const size_t plane = (size_t)n * np;
     const uint32_t tx_bytes = (uint32_t)((size_t)(R0 + R0p) * row_bytes);
     const int lane = threadIdx.x & 31;
     const int NT = blockDim.x;
@@ -331,8 +330,8 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         pr_p1 = p1;
         const int j0 = t * tj;
         const int r0 = (j0 - 2 + n) % n, r1 = (j0 - 1 + n) % n;
-        pr_r[0] = (size_t)r0 * n;
-        pr_r[1] = (size_t)r1 * n;
+        pr_r[0] = (size_t)r0 * np;
+        pr_r[1] = (size_t)r1 * np;
         pr_c[0] = min(R0, n - r0);
         pr_c[1] = min(R0p, n - r1);
     };
@@ -341,7 +340,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
             const int s = is_stage;
             const int pw = pr_pl < 0 ? pr_pl + n : (pr_pl >= n ? pr_pl - n : pr_pl);
             T *dst = ring + (size_t)s * stage_n;
-            T *dpi = dst + (size_t)R0 * n;
+            T *dpi = dst + (size_t)R0 * np;
             const T *gphi = phi_in + (size_t)pw * plane;
             const T *gpi = pi_in + (size_t)pw * plane;
             const uint32_t rb = (uint32_t)row_bytes;
@@ -349,9 +348,9 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
             mbar_arrive_expect_tx(&full[s], tx_bytes);
             const int c0 = pr_c[0], c1 = pr_c[1];
             bulk_g2s(dst, gphi + pr_r[0], (uint32_t)c0 * rb, &full[s]);
-            if (c0 < R0) bulk_g2s(dst + (size_t)c0 * n, gphi, (uint32_t)(R0 - c0) * rb, &full[s]);
+            if (c0 < R0) bulk_g2s(dst + (size_t)c0 * np, gphi, (uint32_t)(R0 - c0) * rb, &full[s]);
             bulk_g2s(dpi, gpi + pr_r[1], (uint32_t)c1 * rb, &full[s]);
-            if (c1 < R0p) bulk_g2s(dpi + (size_t)c1 * n, gpi, (uint32_t)(R0p - c1) * rb, &full[s]);
+            if (c1 < R0p) bulk_g2s(dpi + (size_t)c1 * np, gpi, (uint32_t)(R0p - c1) * rb, &full[s]);
             ++issued;
             if (++is_stage == nstage) is_stage = 0;
             if (++pr_pl > pr_p1 + 1) next_item();
@@ -372,44 +371,45 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     __syncthreads();
 
     const Step<T, BY> step(k);
-    /* the positions as offsets r1 n + kk in an array of level-1 rows (row r1,
-     * first site kk; rows hold n = W nvr sites, so tile position u sits at
-     * n + W u): tile slot s at off0 + s W NT, the halo slot at offh. Where the
+    /* the positions as offsets r1 np + kk in an array of level-1 rows (row r1,
+     * first site kk; rows hold np = W nvr elements, so tile position u sits at
+     * np + W u): tile slot s at off0 + s W NT, the halo slot at offh. Where the
      * tile's positions are no multiple of the threads (!WHOLE), the spare ones
      * repeat the last position and store nothing. */
-    const int npos = tj * (n / W), slot_step = W * NT;
+    const int npos = tj * (np / W), slot_step = W * NT;
     int offs[TB_NTS];
     bool own[TB_NTS];
 #pragma unroll
     for (int s = 0; s < TB_NTS; ++s) {
         const int u = threadIdx.x + s * NT;
         own[s] = WHOLE || u < npos;
-        offs[s] = n + W * (own[s] ? u : npos - 1);
+        offs[s] = np + W * (own[s] ? u : npos - 1);
     }
     using HT = typename Part<T, HW>::V;
     /* whole warps take part in the halo rows (they shuffle) */
-    const bool has_h = HW * (int)(WHOLE ? threadIdx.x : threadIdx.x & ~31) < 2 * n;
-    const bool own_h = HW * (int)threadIdx.x < 2 * n;
-    const int fh = own_h ? HW * (int)threadIdx.x : 2 * n - HW;   /* first halo site, counted over both rows */
-    const int offh = fh + (fh < n ? 0 : tj * n);
+    const bool has_h = HW * (int)(WHOLE ? threadIdx.x : threadIdx.x & ~31) < 2 * np;
+    const bool own_h = HW * (int)threadIdx.x < 2 * np;
+    const int fh = own_h ? HW * (int)threadIdx.x : 2 * np - HW;   /* first halo site, counted over both rows */
+    const int offh = fh + (fh < np ? 0 : tj * np);
     /* the axis-2 neighbours of the vector at shared byte address a: from the
      * neighbouring lanes, at the warp's ends and the row's ends from the row
-     * (periodic). WHOLE: every slot of a thread starts at the same site of its
+     * (periodic; a row's pad holds the images of its first sites, which advance
+     * as those do). WHOLE: every slot of a thread starts at the same site of its
      * row (the slots are whole rows apart) and a row is whole warps. */
     uint32_t from_l[TB_NTS], from_r[TB_NTS];
     int ladj_b[TB_NTS], radj_b[TB_NTS];
 #pragma unroll
     for (int s = 0; s < TB_NTS; ++s) {
-        const int kk = offs[s] % n;
+        const int kk = offs[s] % np;
         from_l[s] = lane == 0 || (!WHOLE && kk == 0);
-        from_r[s] = lane == 31 || (!WHOLE && kk + W == n);
+        from_r[s] = lane == 31 || (!WHOLE && kk + W == np);
         ladj_b[s] = (int)ES * ((kk == 0 ? n : 0) - 1);
-        radj_b[s] = (int)ES * ((kk + W == n ? -n : 0) + W);
+        radj_b[s] = (int)ES * ((kk + W == np ? -n : 0) + W);
     }
     /* the same for the halo share (first site kk_h of its row, HW sites) */
-    const int kk_h = fh % n;
-    const uint32_t from_lh = lane == 0 || (!WHOLE && kk_h == 0), from_rh = lane == 31 || (!WHOLE && kk_h + HW == n);
-    const int ladjh_b = (int)ES * ((kk_h == 0 ? n : 0) - 1), radjh_b = (int)ES * ((kk_h + HW == n ? -n : 0) + HW);
+    const int kk_h = fh % np;
+    const uint32_t from_lh = lane == 0 || (!WHOLE && kk_h == 0), from_rh = lane == 31 || (!WHOLE && kk_h + HW == np);
+    const int ladjh_b = (int)ES * ((kk_h == 0 ? n : 0) - 1), radjh_b = (int)ES * ((kk_h + HW == np ? -n : 0) + HW);
     auto sides = [&](const V &c, uint32_t a, int s, T &left, T &right) {
         const int q = WHOLE ? 0 : s;
         left = __shfl_up_sync(0xffffffffu, last(c), 1);
@@ -418,8 +418,8 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         lds_if(right, a + radj_b[q], from_r[q]);
     };
     const uint32_t ring_a = smem_u32(ring), l1_a = smem_u32(l1);
-    const uint32_t stage_b = ES * (uint32_t)stage_n, slot_b = ES * (uint32_t)slot_n, nb = ES * (uint32_t)n;
-    const uint32_t pi_b = ES * (uint32_t)(R0 * n);
+    const uint32_t stage_b = ES * (uint32_t)stage_n, slot_b = ES * (uint32_t)slot_n, nb = ES * (uint32_t)np;
+    const uint32_t pi_b = ES * (uint32_t)(R0 * np);
     /* the stage and phase parity of round g's plane, advanced once per round */
     int gs = 0, gs_prev = 0;
     uint32_t gph = 0u;
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         /* the slots whose level-2 row is the lattice's (the last tile may hang over) */
         bool keep[TB_NTS];
 #pragma unroll
-        for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own[s] && j0 * n + offs[s] - n < n * n);
+        for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own[s] && j0 * np + offs[s] - np < n * np);
         /* input planes p0 - 2 and p0 - 1: this thread's phi into the register queues */
         if (!bad && acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                 const int m2 = q - 2;
                 const uint32_t L0 = l1_a + ((m2 - p0 + 1) & 1) * slot_b;
                 /* global row j0 - 1 + r1 of plane m2: the tile position's offset from row j0 - 1 */
-                const size_t gbase = ((size_t)m2 * n + (size_t)j0) * n - (size_t)n;
+                const size_t gbase = ((size_t)m2 * n + (size_t)j0) * np - (size_t)np;
                 auto level2 = [&](Slot<V> &x, int s) {
                     const uint32_t ob = L0 + ES * (uint32_t)at(s);
                     const V um = lds<V>(ob - nb);
@@ -592,8 +592,8 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
 
 int sm_count();
 
-/* Geometry of the two-step pass (d = 3, static background, n a multiple of
- * the 16-byte vector, rows of at least one warp: with shorter ones a round's
+/* Geometry of the two-step pass (d = 3, static background, rows of whole
+ * 16-byte vectors (padded, where n is no multiple of one), rows of at least one warp: with shorter ones a round's
  * latency is all there is, 100^3 in float 6.5 us per step against 6.7). A tile is TJ rows; its TJ n / W positions are two per
  * thread, at most 512 threads (so TJ n <= 4096 floats or 2048 doubles), and
  * the halo rows' 2 n / W positions are no more than the threads (TJ >= 4).
@@ -609,12 +609,12 @@ int sm_count();
 bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage, size_t &smem, unsigned &grid,
                       int &parts) {
     const int W = prec == P_FP64 ? 2 : 4;
-    const int n = k.n;
-    if (k.d != 3 || k.expanding || tl != 2 || n % W != 0 || n / W < 32 || n > 1024) return false;
+    const int n = k.n, np = k.pitch;
+    if (k.d != 3 || k.expanding || tl != 2 || np % W != 0 || np / W < 32 || n > 1024) return false;
     if (prec == P_FP64 && !k.dx2_pow2 && !k.dx2_pair) return false;
-    const size_t row = (size_t)n * (prec == P_FP64 ? 8 : 4);
+    const size_t row = (size_t)np * (prec == P_FP64 ? 8 : 4);
     const size_t budget = 227 * 1024 - 1024 - TB_HDR;   /* dynamic share of 227 KB, room for the static variables */
-    const int nv = n / W;
+    const int nv = np / W;
     const long long slots = sm_count();
     double best = 0.0;
     for (int t = 4; t <= 32 && t * nv <= TB_NTS * TB_MAXT; ++t) {
@@ -623,7 +623,7 @@ bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage
         const long long ntiles = (n + t - 1) / t;
         const int per_sched = (t * nv + 255) / 256;   /* warps per scheduler, two vectors each */
         /* rows of whole warps in whole tiles save the masks and per-slot wraps (launch below) */
-        const bool whole = nv % 32 == 0 && n % t == 0 && t * nv % 64 == 0;
+        const bool whole = np == n && nv % 32 == 0 && n % t == 0 && t * nv % 64 == 0;
         const double round = (whole ? 1.0 : 1.15) + (prec == P_FP64 ? 0.05 : 0.036) * (4.0 * per_sched + (2 * nv + 127) / 128);
         for (long long w = 1; w <= 8; ++w) {
             const long long P = std::min<long long>(w * slots / ntiles, n / 4);
@@ -654,11 +654,11 @@ cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *ph
     unsigned grid;
     if (!step3tb_geometry(k, prec, tl, tj, nstage, smem, grid, parts)) return cudaErrorInvalidValue;
     const int W = prec == P_FP64 ? 2 : 4;
-    const int npos = tj * (k.n / W);
+    const int npos = tj * (k.pitch / W);
     const int nc = (npos + 64 - 1) / 64 * 32;
     /* rows of whole warps, whole tiles, every thread two positions: the halo rows'
      * 2 n sites then spread as 1, 2 (float: 4) per thread where that comes out even */
-    const bool whole = (k.n / W) % 32 == 0 && k.n % tj == 0 && npos == 2 * nc;
+    const bool whole = k.pitch == k.n && (k.n / W) % 32 == 0 && k.n % tj == 0 && npos == 2 * nc;
     auto go = [&](auto t, auto by, auto hw, auto wh) -> cudaError_t {
         using T = decltype(t);
         auto fn = k_step3_t2<T, decltype(by)::value, decltype(hw)::value, decltype(wh)::value>;
