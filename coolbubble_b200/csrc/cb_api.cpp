@@ -323,9 +323,10 @@ int alloc_handle(const cb_params *p, cb_handle **out) {
 void destroy_handle(cb_handle *h) {
     if (!h) return;
     finish_writer(h);
-    for (auto &row : h->graph)
-        for (auto &g : row)
-            if (g) cudaGraphExecDestroy(g);
+    for (auto &plane : h->graph)
+        for (auto &row : plane)
+            for (auto &g : row)
+                if (g) cudaGraphExecDestroy(g);
     /* every release is ordered after the run's queued work on its own stream */
     auto dfree = [&](void *p) {
         if (p) cudaFreeAsync(p, h->stream);
@@ -499,7 +500,7 @@ bool graphs_wanted(const cb_handle *h) {
 /* CB_OK: GRAPH_STEPS steps queued; 1: graphs unavailable (launch plainly); < 0: error */
 int replay_step_graph(cb_handle *h) {
     const int i = h->cphi, j = h->cpi;
-    cudaGraphExec_t &ex = h->graph[i][j];
+    cudaGraphExec_t &ex = h->graph[i][j][h->steps_done & 1];
     if (!ex) {
         StepConst k = h->k;
         k.want_local = 0;
@@ -513,6 +514,7 @@ int replay_step_graph(cb_handle *h) {
         }
         int ci = i, cj = j;
         for (int q = 0; q < GRAPH_STEPS && e == cudaSuccess; ++q) {
+            k.odd = (int)((h->steps_done + q) & 1);
             e = launch_step(h->prec, k, h->expanding, sums, h->phi[ci], h->pi[cj], h->phi[1 - ci], h->pi[1 - cj],
                             h->loc[0], h->loc[1], h->loc[2], h->st, h->partials, h->stream);
             ci = 1 - ci;
@@ -565,8 +567,13 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
         if (ms_ok && !h->multi_off && plain_left >= 2) {
             const int m = std::min(plain_left, MULTI_STEP_MAX);
             const int i = h->cphi, j = h->cpi;
-            e = launch_step3_ms(h->prec, h->k, m, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j], h->st,
-                                h->partials, h->stream);
+            StepConst km = h->k;
+            km.odd = (int)(h->steps_done & 1);
+            e = step3df_applies(km, h->prec)
+                    ? launch_step3_df(h->prec, km, m, true, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j], h->st,
+                                      h->partials, h->stream)
+                    : launch_step3_ms(h->prec, km, m, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j], h->st,
+                                      h->partials, h->stream);
             if (e == cudaErrorNotSupported) {
                 cudaGetLastError();
                 h->multi_off = true;   /* steps one launch each from now on */
@@ -634,6 +641,7 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
         const int sums = want ? 2 : (h->expanding ? 1 : 0);
         StepConst k = h->k;
         k.want_local = local ? 1 : 0;
+        k.odd = (int)(h->steps_done & 1);
         const int i = h->cphi, j = h->cpi;
         e = launch_step(h->prec, k, h->expanding, sums, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j],
                         h->loc[0], h->loc[1], h->loc[2], h->st, h->partials, h->stream);

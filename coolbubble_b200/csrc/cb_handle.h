@@ -57,8 +57,8 @@ struct cb_handle {
     cudaEvent_t ev[2] = {nullptr, nullptr};
     cb::FftState *fft = nullptr;
     cb::SnapshotWriter *writer = nullptr;
-    /* replayable chains of plain steps (small lattices), by (cphi, cpi) at their start */
-    cudaGraphExec_t graph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
+    /* replayable chains of plain steps (small lattices), by (cphi, cpi, step parity) at their start */
+    cudaGraphExec_t graph[2][2][2] = {};
     bool graphs_off = false;
     bool multi_off = false;  /* multi-step launches unavailable (or CB_MULTI_STEP=0) */
     std::string err;

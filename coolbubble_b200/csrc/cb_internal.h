@@ -86,6 +86,8 @@ struct StepConst {
     int alpha, expanding;
     int want_local;
     int force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
+    int odd;            /* the step's index is odd: expanding steps march the planes in turn forwards and
+                           backwards */
     int temporal;       /* steps per pass for static float 3-D lattices (1: no temporal blocking) */
 };
 
@@ -150,6 +152,15 @@ cudaError_t launch_step3(int prec, const StepConst &k, bool drift_first, int sum
                          DevState *st, double *partials, cudaStream_t s);
 cudaError_t launch_step3_ms(int prec, const StepConst &k, int nsteps, void *phi_a, void *pi_a, void *phi_b,
                             void *pi_b, DevState *st, double *partials, cudaStream_t s);
+
+/* Plain steps of an expanding background (cb_step3_df.cu): one step, or with
+ * `cooperative` nsteps >= 1 of them in one launch (A = the fields now, B = the
+ * other buffers; the fields end in B for odd nsteps). cudaErrorNotSupported
+ * where the kernel does not apply, or its blocks cannot all be resident. */
+cudaError_t launch_step3_df(int prec, const StepConst &k, int nsteps, bool cooperative, void *phi_a, void *pi_a,
+                            void *phi_b, void *pi_b, DevState *st, double *partials, cudaStream_t s);
+bool step3df_applies(const StepConst &k, int prec);
+size_t step3df_partial_rows(const StepConst &k, int prec);
 
 /* TL steps per pass, static float 3-D lattices (cb_step3_tb.cu). */
 bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage, size_t &smem, unsigned &grid,

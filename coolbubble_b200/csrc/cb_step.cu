@@ -473,6 +473,7 @@ size_t step_blocks(const StepConst &k) {
         size_t sm;
         unsigned g3;
         if (step3_geometry(k, prec, tj, ns, sm, g3)) b = std::max(b, step3_partial_rows(k, prec));
+        if (step3df_applies(k, prec)) b = std::max(b, step3df_partial_rows(k, prec));
     }
     if (k.d <= 2) b = std::max(b, step2_blocks(k));
     return b;
@@ -486,6 +487,9 @@ cudaError_t launch_step(int prec, const StepConst &k, bool drift_first, int sums
     int tj, ns;
     size_t sm;
     unsigned g3;
+    if (drift_first && sums == SUM_FRIEDMANN && step3df_applies(k, prec))
+        return launch_step3_df(prec, k, 1, false, const_cast<void *>(phi_in), const_cast<void *>(pi_in), phi_out,
+                               pi_out, st, partials, s);
     if (step2_applies(k, prec, drift_first))
         return launch_step2(prec, k, sums, phi_in, pi_in, phi_out, pi_out, loc_ek, loc_eg, loc_ep, st, partials, s);
     /* padded rows in float: the reporting step stays with the generic kernel, whose

@@ -959,28 +959,34 @@ cudaError_t launch_step3(int prec, const StepConst &k, bool df, int sums, const 
     return cudaGetLastError();
 }
 
-/* nsteps >= 1 drift-first float steps with the Friedmann sums in one
- * cooperative launch (A = the fields now, B = the other buffers; the fields
- * end in B for odd nsteps). cudaErrorNotSupported where the staged kernel
- * does not apply or its blocks cannot all be resident (the caller then
- * launches the steps one by one). */
+static bool step3_one_round(const StepConst &k, int prec) {
+    int tj, nstage, parts;
+    size_t smem;
+    unsigned grid;
+    return k.expanding && k.d == 3 && step3_geometry_parts(k, prec, tj, nstage, smem, grid, parts) &&
+           (long long)((k.n + tj - 1) / tj) * parts <= (long long)grid;
+}
+
+/* nsteps >= 1 drift-first steps with the Friedmann sums in one cooperative
+ * launch (A = the fields now, B = the other buffers; the fields end in B for
+ * odd nsteps). cudaErrorNotSupported where the staged kernel does not apply or
+ * its blocks cannot all be resident (the caller then launches the steps one by
+ * one). Only where a step is one round of items (every block one item): there
+ * the launch gap and the ramp of each step are what a multi-step launch saves
+ * (float, 256^3: 0.0540 -> 0.0524 ms per step, 128^3: 0.0142 -> 0.0125). */
 template <typename T>
 cudaError_t launch_step3_ms_t(int prec, const StepConst &k, int nsteps, void *phi_a, void *pi_a, void *phi_b,
                               void *pi_b, DevState *st, double *partials, cudaStream_t s) {
     int tj, nstage, parts;
     size_t smem;
     unsigned grid;
-    if (!k.expanding || k.d != 3 || nsteps < 1 || !step3_geometry_parts(k, prec, tj, nstage, smem, grid, parts))
+    if (nsteps < 1 || !step3_one_round(k, prec) || !step3_geometry_parts(k, prec, tj, nstage, smem, grid, parts))
         return cudaErrorNotSupported;
-    /* only where a step is one round of items (every block one item): there
-     * the launch gap and the ramp of each step are what a multi-step launch
-     * saves (256^3: 0.0540 -> 0.0524 ms per step, 128^3: 0.0142 -> 0.0125);
-     * with several rounds per step one launch per step measured faster
-     * (384^3: 0.165 against 0.179 ms, 512^3: 0.393 against 0.404) */
-    if ((long long)((k.n + tj - 1) / tj) * parts > (long long)grid) return cudaErrorNotSupported;
     const bool rag = k.pitch != k.n;
-    auto fn = k.alpha == 1 ? (rag ? k_step3<T, true, SUM_FRIEDMANN_EG, true, true> : k_step3<T, true, SUM_FRIEDMANN_EG, false, true>)
-                           : (rag ? k_step3<T, true, SUM_FRIEDMANN, true, true> : k_step3<T, true, SUM_FRIEDMANN, false, true>);
+    auto fn = k.alpha == 1 ? (rag ? k_step3<T, true, SUM_FRIEDMANN_EG, true, true>
+                                  : k_step3<T, true, SUM_FRIEDMANN_EG, false, true>)
+                           : (rag ? k_step3<T, true, SUM_FRIEDMANN, true, true>
+                                  : k_step3<T, true, SUM_FRIEDMANN, false, true>);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;

@@ -46,6 +46,7 @@
 
 #include "cb_internal.h"
 #include "cb_launch.cuh"
+#include "cb_march.cuh"
 #include "cb_step_common.cuh"
 #include "cb_tma.cuh"
 
@@ -57,95 +58,6 @@ constexpr int TB_MAXT = 512;             /* threads per block (all of them compu
 constexpr int TB_NTS = 2;                 /* tile positions per thread */
 constexpr int TB_HDR = 256;               /* full[nstage] mbarriers (nstage <= 8) */
 constexpr int TB_IQ = 8;
-
-/* block-wide barrier (bar.red over all threads), returning whether any
- * thread passed true */
-__device__ __forceinline__ bool tb_any(bool x) { return __syncthreads_or(x ? 1 : 0) != 0; }
-
-/* shared-memory accesses by 32-bit shared address */
-template <typename V>
-__device__ __forceinline__ V lds(uint32_t a);
-template <>
-__device__ __forceinline__ float lds<float>(uint32_t a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-template <>
-__device__ __forceinline__ float2 lds<float2>(uint32_t a) {
-    float2 v;
-    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-    return v;
-}
-template <>
-__device__ __forceinline__ float4 lds<float4>(uint32_t a) {
-    float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
-}
-template <>
-__device__ __forceinline__ double lds<double>(uint32_t a) {
-    double v;
-    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-    return v;
-}
-template <>
-__device__ __forceinline__ double2 lds<double2>(uint32_t a) {
-    double2 v;
-    asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void sts(uint32_t a, float v) {
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, const float2 &v) {
-    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, const float4 &v) {
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                 : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, double v) {
-    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void sts(uint32_t a, const double2 &v) {
-    asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
-}
-/* v = shared value at a where pred != 0 (a predicated load: no branch) */
-__device__ __forceinline__ void lds_if(float &v, uint32_t a, uint32_t pred) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}"
-                 : "+f"(v)
-                 : "r"(a), "r"(pred));
-}
-__device__ __forceinline__ void lds_if(double &v, uint32_t a, uint32_t pred) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p ld.shared.f64 %0, [%1];\n\t}"
-                 : "+d"(v)
-                 : "r"(a), "r"(pred));
-}
-
-/* the sites of 1, 2 or 4 consecutive positions, by their count */
-template <typename T, int N>
-struct Part;
-template <>
-struct Part<float, 1> { using V = float; };
-template <>
-struct Part<float, 2> { using V = float2; };
-template <>
-struct Part<float, 4> { using V = float4; };
-template <>
-struct Part<double, 1> { using V = double; };
-template <>
-struct Part<double, 2> { using V = double2; };
-__device__ __forceinline__ float first(float v) { return v; }
-__device__ __forceinline__ float first(const float2 &v) { return v.x; }
-__device__ __forceinline__ float first(const float4 &v) { return v.x; }
-__device__ __forceinline__ double first(double v) { return v; }
-__device__ __forceinline__ double first(const double2 &v) { return v.x; }
-__device__ __forceinline__ float last(float v) { return v; }
-__device__ __forceinline__ float last(const float2 &v) { return v.y; }
-__device__ __forceinline__ float last(const float4 &v) { return v.w; }
-__device__ __forceinline__ double last(double v) { return v; }
-__device__ __forceinline__ double last(const double2 &v) { return v.y; }
 
 /* One leapfrog step on the static background: pi' = pi + dt F(phi), phi' =
  * phi + dt pi' (bubble.cpp:716-743, 853-856, 867-870 with a = 1), for the
@@ -432,7 +344,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     };
     /* round g: wait for input plane g; false (and the abort flag) if the wait ran out */
     auto acquire = [&]() -> bool {
-        const bool ok = abort_flag == 0 && mbar_wait(&full[gs], gph, WAIT_LIMIT);
+        const bool ok = mbar_wait(&full[gs], gph, WAIT_LIMIT);   /* a wait that ran out is voted on below */
         if (!ok) atomicExch(&abort_flag, 1);
         return ok;
     };
