@@ -31,8 +31,8 @@
  *  - What bounds it: the latency of a round (load, two dependent updates, a
  *    barrier) over 16 warps, ncu on 256^3: float FMA pipe 62 % busy, issue 55 %;
  *    double FP64 pipe 36 %, issue 50 %; DRAM 41-47 %. us per step, one step per
- *    pass -> here: 192^3 float 19.0 -> 17.1, 256^3 50.0 -> 27.9, 512^3 336 ->
- *    197, 256^3 double 89 -> 63, 192^3 double 44.7 -> 29.9.
+ *    pass -> here: 192^3 float 19.0 -> 16.2, 256^3 50.0 -> 27.3, 512^3 336 ->
+ *    193, 256^3 double 89 -> 60, 192^3 double 44.7 -> 28.9.
  *  - Waits are bounded (clock64 limit, sleeping retries); a timed-out block
  *    records an error word; consumer warps leave together (a vote in the
  *    per-round barrier).
@@ -71,16 +71,16 @@ struct Step;
  * half is rounded on its own) */
 template <int BY>
 struct Step<float, BY> {
-    F2 idx2, dt, nc2, c3, nc4;
+    F2 idx2, dt, nc2, c3, nc4, m2;
     __device__ __forceinline__ explicit Step(const StepConst &k)
         : idx2(f2_splat(k.inv_dx2f)), dt(f2_splat(k.dtf)), nc2(f2_splat(-k.c2f)), c3(f2_splat(k.c3f)),
-          nc4(f2_splat(-k.c4f)) {}
+          nc4(f2_splat(-k.c4f)), m2(f2_splat(-2.f)) {}
     __device__ __forceinline__ void pair(F2 cc, F2 umm, F2 upp, F2 imm, F2 ipp, F2 kmm, F2 kpp, F2 pp, F2 &phi2,
                                          F2 &pi2) const {
-        const F2 two = f2_add(cc, cc);
-        const F2 t0 = f2_add(f2_sub(ipp, two), imm);
-        const F2 t1 = f2_add(f2_sub(upp, two), umm);
-        const F2 t2 = f2_add(f2_sub(kpp, two), kmm);
+        /* x - 2 c in one rounding: 2 c is exact */
+        const F2 t0 = f2_add(f2_fma(cc, m2, ipp), imm);
+        const F2 t1 = f2_add(f2_fma(cc, m2, upp), umm);
+        const F2 t2 = f2_add(f2_fma(cc, m2, kpp), kmm);
         const F2 lap = f2_add(f2_add(t0, t1), t2);
         /* -V'(f)/f = -(c2 + f (-c3 + f c4)) with every operand negated: the
          * exact negation of the one-step kernel's rounded h (round to nearest
@@ -131,10 +131,10 @@ struct Step<double, BY> {
     __device__ __forceinline__ void operator()(double c, double um, double up, double im, double ip, double left,
                                                double right, double pv, double &phi, double &pi) const {
         using A = Ar<double>;
-        const double two = A::add(c, c);
-        const double t0 = A::add(A::sub(ip, two), im);
-        const double t1 = A::add(A::sub(up, two), um);
-        const double t2 = A::add(A::sub(right, two), left);
+        /* x - 2 c in one rounding: 2 c is exact */
+        const double t0 = A::add(__fma_rn(c, -2.0, ip), im);
+        const double t1 = A::add(__fma_rn(c, -2.0, up), um);
+        const double t2 = A::add(__fma_rn(c, -2.0, right), left);
         const double lap = A::add(A::add(t0, t1), t2);
         pi = A::add(pv, A::mul(k.dt, A::sub(over_dx2<BY>(k, lap), dV<double>(k, c))));
         phi = A::add(c, A::mul(k.dt, pi));
@@ -569,7 +569,10 @@ cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *ph
     const int npos = tj * (k.pitch / W);
     const int nc = (npos + 64 - 1) / 64 * 32;
     /* rows of whole warps, whole tiles, every thread two positions: the halo rows'
-     * 2 n sites then spread as 1, 2 (float: 4) per thread where that comes out even */
+     * 2 n sites then spread as 1, 2 (float: 4) per thread where that comes out even.
+     * Other rows spread them as one pair of floats or one double per thread where the
+     * threads suffice (250^3 float 29.3 us per step with whole vectors on some of the
+     * warps, 28.4 with pairs, 31.5 site by site; 200^3 double 34.9 -> 33.7) */
     const bool whole = k.pitch == k.n && (k.n / W) % 32 == 0 && k.n % tj == 0 && npos == 2 * nc;
     auto go = [&](auto t, auto by, auto hw, auto wh) -> cudaError_t {
         using T = decltype(t);
@@ -587,11 +590,11 @@ cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *ph
     constexpr integral_constant<int, 4> four{};
     if (prec != P_FP64) {
         constexpr integral_constant<int, BY_MUL> mul{};
-        if (!whole) return go(0.f, mul, four, no);
+        if (!whole) return k.pitch <= nc ? go(0.f, mul, two, no) : go(0.f, mul, four, no);
         return 2 * k.n == nc ? go(0.f, mul, one, yes) : k.n == nc ? go(0.f, mul, two, yes) : go(0.f, mul, four, yes);
     }
     auto doubles = [&](auto by) {
-        if (!whole) return go(0.0, by, two, no);
+        if (!whole) return 2 * k.pitch <= nc ? go(0.0, by, one, no) : go(0.0, by, two, no);
         return 2 * k.n == nc ? go(0.0, by, one, yes) : go(0.0, by, two, yes);
     };
     return k.dx2_pow2 ? doubles(integral_constant<int, BY_MUL>{}) : doubles(integral_constant<int, BY_PAIR>{});
