@@ -930,14 +930,14 @@ int cb_get_fields_f32(cb_handle *h, float *phi, float *pi, float *ekin, float *e
             continue;
         }
         const void *from = src[f];
-        if (h->prec == P_FP64) {
+        if (h->prec == P_FP64) {   /* through the staging buffer, in stream order */
             e = launch_convert(P_FP64, P_FP32, src[f], h->tmp, h->N, h->stream);
             from = h->tmp;
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst[f], from, h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         if (e != cudaSuccess) return cuda_fail(h, e, "downloading a field");
     }
+    if ((r = sync(h, "downloading the fields")) != CB_OK) return r;
     return CB_OK;
 }
 

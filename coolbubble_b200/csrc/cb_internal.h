@@ -4,6 +4,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -143,6 +144,21 @@ cudaError_t launch_step2(int prec, const StepConst &k, int sums, const void *phi
 int step2tb_steps(const StepConst &k, int prec, int left, bool sums);
 cudaError_t launch_step2_tb(int prec, const StepConst &k, int steps, bool sums, const void *phi_in, const void *pi_in,
                             void *phi_out, void *pi_out, DevState *st, double *partials, cudaStream_t s);
+
+/* Many static d = 2 lattices of one precision and kind per launch: steps at a
+ * time (batch2_steps of the `left` to come), the last with sums into record
+ * `event` of each (< 0: none). flip: which of a member's buffers hold the
+ * fields now; partials: batch2_partial_rows rows. ns: the members' n. */
+struct Batch2Member {
+    StepConst k;
+    void *phi[2], *pi[2];
+    DevState *st, *records;
+};
+int batch2_kind(const StepConst &k, int prec);   /* members of a launch share it: form of the rows, division by dx^2 */
+int batch2_steps(const std::vector<int> &ns, int prec, int kind, int left);
+size_t batch2_partial_rows(const std::vector<int> &ns, int prec, int kind, int steps);
+cudaError_t launch_step2_batch(int prec, int kind, const Batch2Member *members, const std::vector<int> &ns, int steps,
+                               int flip, int event, double *partials, cudaStream_t s);
 
 /* d = 3 kernel with TMA-staged row tiles (cb_step3.cu). */
 bool step3_geometry(const StepConst &k, int prec, int &tj, int &nstage, size_t &smem, unsigned &grid);

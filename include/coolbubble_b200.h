@@ -281,11 +281,9 @@ int cb_step_static_noalloc(const cb_params *p, const void *phi_in, const void *p
 
 /* No counterpart in the reference, which runs one lattice per process
  * (main.cpp:45-50). Groups existing runs (their handles stay valid and keep
- * owning their memory). Two-dimensional static runs whose fields fit in the
- * shared memory of a thread-block cluster (float: n <= 512, double: n <= 256)
- * are stepped resident in shared memory, one launch per size class, with the
- * CTA size chosen by timing candidates once per class (cached per process);
- * the other members step on their own streams, concurrently. */
+ * owning their memory). Two-dimensional static runs are stepped in batches,
+ * many lattices and several steps per launch; the other members step on their
+ * own streams, concurrently. */
 typedef struct cb_ensemble cb_ensemble;
 int cb_ensemble_create(int count, cb_handle *const *members, cb_ensemble **out);
 
@@ -293,8 +291,10 @@ int cb_ensemble_create(int count, cb_handle *const *members, cb_ensemble **out);
  * sums_every-th step of member m goes to out[m * (nsteps / sums_every) + j]. */
 int cb_ensemble_step(cb_ensemble *e, int nsteps, int sums_every, cb_sums *out);
 
-/* How member m is stepped: the cluster size of its resident class (1..16)
- * and the CTA size the autotuner chose, or 0, 0 when it steps on its own. */
+/* The size class of a batched member -- the shares of 200 KB (1, 2, 4, 8, 16)
+ * that three of its fields fill in whole rows -- and the threads of a block;
+ * 0, 0 for members larger than a class, with other rows, or stepped on their
+ * own. */
 int cb_ensemble_member_plan(cb_ensemble *e, int m, int *cluster, int *threads);
 
 int cb_ensemble_destroy(cb_ensemble *e);

@@ -1,0 +1,45 @@
+"""Ensembles stepped in batches: members of every form of row, sizes mixed in
+one launch, against their solo runs, bit for bit in the fields."""
+import numpy as np
+import pytest
+
+from ic_helpers import smooth_noise
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32c"])
+def test_batched_members_equal_their_solo_runs(prec):
+    import coolbubble_b200 as cb
+    from coolbubble_b200.ensemble import Ensemble
+    # whole rows of 8, 16, 32 lanes; vectors; site by site; dx^2 that divides in one, two operations and neither
+    specs = [(32, 4.0), (64, 8.0), (128, 16.0), (64, 6.4), (200, 20.0), (256, 32.0), (101, 10.1), (502, 30.0), (5, 0.5)]
+    made = []
+    for i, (n, L) in enumerate(specs):
+        p = cb.make_params(2, n, L, 2.0 + i % 3, 0.1 * L / n, precision=prec, memorysave=1)
+        made.append((p, 0.3 + smooth_noise(2, n, 0.1, seed=i), smooth_noise(2, n, 0.05, seed=90 + i)))
+    mix = [cb.Bubble(*m) for m in made]
+    solo = [cb.Bubble(*m) for m in made]
+    mix[2].step(3, sums=False)   # another buffer state than the others'
+    solo[2].step(3, sums=False)
+    ens = Ensemble(mix)
+    for nsteps, every in ((7, 0), (85, 40), (1, 1), (40, 13)):
+        lines = ens.step(nsteps, every)
+        for i, s in enumerate(solo):
+            ref, done = [], 0
+            while every and done + every <= nsteps:
+                ref.append(s.step(every, sums=True))
+                done += every
+            if done < nsteps:
+                s.step(nsteps - done, sums=False)
+            assert len(lines[i]) == len(ref)
+            for got, want in zip(lines[i], ref):
+                assert got["t"] == want["t"] and got["a"] == want["a"]
+                for key in ("etot", "ekin", "egrad", "epot", "etot_var", "avphi_var"):
+                    # the same terms, added in double in another order
+                    assert abs(got[key] - want[key]) <= s.N * 2.0 ** -52 * abs(want[key]), (i, key)
+    for i, (m, s) in enumerate(zip(mix, solo)):
+        fa, fb = m.fields(), s.fields()
+        np.testing.assert_array_equal(fa["phi"], fb["phi"], err_msg=str(specs[i]))
+        np.testing.assert_array_equal(fa["pi"], fb["pi"], err_msg=str(specs[i]))
+        assert m.sums()["t"] == s.sums()["t"] and m.counters()[1] == s.counters()[1]

@@ -12,6 +12,7 @@ POSITIVE = ("etot", "ekin", "egrad", "epot", "etot_var", "ekin_var", "egrad_var"
 
 @pytest.mark.parametrize("d,n,L", [
     (2, 5, 0.5),          # smaller than a tile's halo: coordinates wrap several times
+    (2, 16, 2.0), (2, 32, 3.2), (2, 128, 16.0),   # a whole row on 8, 16 or 32 lanes
     (2, 64, 8.0), (2, 101, 12.625), (2, 250, 25.0),   # vectors, odd rows (site by site), double vectors only
     (2, 512, 32.0), (2, 1000, 100.0), (2, 1031, 103.1),   # several tiles, tiles over the end, more tiles than blocks
     (2, 502, 30.0),       # dx^2 has no two-operation division: the compiler's divides
