@@ -69,9 +69,6 @@ struct StepConst {
     int d, n;
     int ni, nj, nk;     /* extents mapped onto (march axis, tile rows, tile columns) */
     int cz;             /* planes per block along the march axis (generic d = 3 kernel) */
-    int pitch;          /* elements from a row of the last axis to the next: n, or (d = 3 runs) n rounded
-                           up to whole 16-byte vectors. The pad holds the periodic images of the row's
-                           first sites: every kernel that writes phi or pi keeps them equal */
     double dt;
     double c2, c3, c4;  /* V'(f) = c2 f - c3 f^2 + c4 f^3, coefficients as bubble.cpp:76 forms them */
     double v2, v3, v4, dv; /* V(f) = v2 f^2 - v3 f^3 + v4 f^4 + DeltaV (bubble.cpp:71) */
@@ -80,16 +77,20 @@ struct StepConst {
     float c2f, c3f, c4f, v2f, v3f, v4f, dvf;
     float dtf, dxf, dx2f, inv_dx2f;
     double dx, dx2, inv_dx2;
-    double inv_dx2_lo;  /* 1/dx2 - inv_dx2, rounded */
     int dx2_pow2;
-    int dx2_pair;       /* fma(x, inv_dx2, x inv_dx2_lo) is x / dx2 rounded (reciprocal_pair, cb_api.cpp) */
     double dxLD, mpl;
     int alpha, expanding;
     int want_local;
     int force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
+    int temporal;       /* steps per pass for static float 3-D lattices (1: no temporal blocking) */
+    /* fields below: behind those that the kernels load in groups of 16 bytes */
+    int pitch;          /* elements from a row of the last axis to the next: n, or (d = 3 runs) n rounded
+                           up to whole 16-byte vectors. The pad holds the periodic images of the row's
+                           first sites: every kernel that writes phi or pi keeps them equal */
     int odd;            /* the step's index is odd: expanding steps march the planes in turn forwards and
                            backwards */
-    int temporal;       /* steps per pass for static float 3-D lattices (1: no temporal blocking) */
+    int dx2_pair;       /* fma(x, inv_dx2, x inv_dx2_lo) is x / dx2 rounded (reciprocal_pair, cb_api.cpp) */
+    double inv_dx2_lo;  /* 1/dx2 - inv_dx2, rounded */
 };
 
 /* The checks of one line from its energies, in double and in this order (the
@@ -117,7 +118,10 @@ enum Prec { P_FP64 = 0, P_FP32 = 1 };
  * SUM_FRIEDMANN_EG: the Friedmann sums with the gradient energy (conformal
  * time, alpha = 1); the staged d = 3 kernel takes it as its own variant so
  * the choice is made at compile time. */
-enum SumMode { SUM_NONE = 0, SUM_FRIEDMANN = 1, SUM_FULL = 2, SUM_FRIEDMANN_EG = 3 };
+/* SUM_LINE: every box average and no local energy arrays -- the staged d = 3
+ * kernel's own variant in double, with the sums' terms formed in fewer
+ * operations than the arrays' values. */
+enum SumMode { SUM_NONE = 0, SUM_FRIEDMANN = 1, SUM_FULL = 2, SUM_FRIEDMANN_EG = 3, SUM_LINE = 4 };
 
 /* sums: 0 none, 1 only what the Friedmann update needs, 2 every box average */
 cudaError_t launch_step(int prec, const StepConst &k, bool drift_first, int sums, const void *phi_in,

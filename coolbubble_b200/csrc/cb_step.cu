@@ -492,10 +492,7 @@ cudaError_t launch_step(int prec, const StepConst &k, bool drift_first, int sums
                                pi_out, st, partials, s);
     if (step2_applies(k, prec, drift_first))
         return launch_step2(prec, k, sums, phi_in, pi_in, phi_out, pi_out, loc_ek, loc_eg, loc_ep, st, partials, s);
-    /* padded rows in float: the reporting step stays with the generic kernel, whose
-     * sums are compensated per site (the staged kernel's averages are plain pair sums) */
-    const bool plain_sums = k.pitch != k.n && prec == P_FP32 && sums == SUM_FULL;
-    if (!k.force_generic && !plain_sums && step3_geometry(k, prec, tj, ns, sm, g3))
+    if (!k.force_generic && step3_geometry(k, prec, tj, ns, sm, g3))
         return launch_step3(prec, k, drift_first, sums, phi_in, pi_in, phi_out, pi_out, loc_ek, loc_eg, loc_ep, st,
                             partials, s);
     if (prec == P_FP64)

@@ -186,7 +186,11 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     using VT = typename Vec<T>::V;
     constexpr int W = Vec<T>::W;
     constexpr bool UNI = DF || SUMS != SUM_NONE;       /* consumers leave together */
-    constexpr int NS = SUMS == SUM_FULL ? NSUM : 3;    /* sums carried (S_EK, S_EP, S_EG first) */
+    constexpr bool FULL = SUMS == SUM_FULL || SUMS == SUM_LINE;
+    constexpr int NS = FULL ? NSUM : 3;                /* sums carried (S_EK, S_EP, S_EG first) */
+    /* float with padded rows: the full sums in double per vector (250^3: 69 us; the
+     * generic kernel, which compensates its sums per site, 180) */
+    constexpr bool DSUM = RAG && SUMS == SUM_FULL && std::is_same<T, float>::value;
     extern __shared__ __align__(128) unsigned char smraw[];
     const int n = NV ? NV * W : k.n, np = RAG ? k.pitch : n;   /* sites and elements of a row */
     const int tj = NV ? NV_TILE / NV : tj_;
@@ -252,6 +256,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     Acc<T> acc[NSUM];
     AccF2 kacc[NSUM];   /* float path: the compensated sums (energies) */
     F2 pacc[NSUM];      /* float path: plain pair sums (averages; squares by fused multiply-add) */
+    double dacc[NSUM];  /* DSUM, SUM_LINE */
 
     if (warp == CW) {
         /* ---- producer warp: lane 0 takes items from the queue and issues the
@@ -358,12 +363,19 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             const T dt = kc<T>(k.dt, k.dtf);
             const T p = DF ? (T)cs->drift_p : (T)1;
             const T dx2 = kc<T>(k.dx2, k.dx2f), inv_dx2 = kc<T>(k.inv_dx2, k.inv_dx2f);
-            const bool dx2_pow2 = std::is_same<T, float>::value || k.dx2_pow2 != 0;
             const T half = (T)0.5;
+            /* flap / dx^2, correctly rounded (see over_dx2; the pair covers powers of two too) */
+            const bool dx2_pair = k.dx2_pair != 0;
+            auto over = [&](T x) -> T {
+                if constexpr (std::is_same<T, double>::value)
+                    return dx2_pair ? over_dx2<BY_PAIR>(k, x) : A::div(x, dx2);
+                else
+                    return A::mul(x, inv_dx2);
+            };
             auto grad = [&](T dphi) -> T { return adx_pow2 ? A::mul(dphi, inv_adx) : A::div(dphi, adx); };
             const int nvec_row = np / W;
             const int row_step = NC / nvec_row, vec_step = NC % nvec_row;
-            constexpr bool want_eg = SUMS == SUM_FULL || SUMS == SUM_FRIEDMANN_EG;
+            constexpr bool want_eg = FULL || SUMS == SUM_FRIEDMANN_EG;
             /* float steps run in packed f32x2 pairs, with or without sums */
             constexpr bool PACKED = std::is_same<T, float>::value;
             /* packed-pair constants of the f32x2 path (unused otherwise) */
@@ -373,6 +385,9 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             const F2 P_V2 = f2_splat(k.v2f), P_NV3 = f2_splat(-k.v3f), P_V4 = f2_splat(k.v4f), P_DV = f2_splat(k.dvf);
             /* gradient energy 0.5 |grad phi|^2 / (a dx)^2 as one product with the sum of squared differences */
             const F2 P_EG = f2_splat((float)(0.5 * (double)inv_adx * (double)inv_adx)), P_VW = f2_splat((float)vel_w);
+            const F2 P_IA = f2_splat((float)inv_adx), P_HALF = f2_splat(0.5f);
+            /* SUM_LINE: 0.5 / (a dx)^2 */
+            const double eg_w = SUMS == SUM_LINE ? __ddiv_rn(0.5, __dmul_rn(cs->adx, cs->adx)) : 0.0;
             /* wait for the ring position under cursor c to land */
             auto acquire = [&](const Cursor &c) -> bool {
                 const bool ok = abort_flag == 0 && mbar_wait(&full[c.s], c.ph, WAIT_LIMIT);
@@ -448,6 +463,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                         acc[s] = Acc<T>{};
                         kacc[s] = AccF2{};
                         pacc[s] = f2_splat(0.f);
+                        dacc[s] = 0.0;
                     }
                 }
                 /* cm, c0, cp: cursors of planes i - 1, i, i + 1 */
@@ -541,8 +557,13 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                                 F2 eg = f2_splat(0.f);
                                 if constexpr (want_eg) {
                                     /* forward differences: x <- axis 1, y <- axis 0, z <- axis 2 (bubble.cpp:794-801) */
-                                    const F2 gx = f2_sub(upp, cc), gy = f2_sub(ipp, cc), gz = f2_sub(kpp, cc);
-                                    eg = f2_mul(P_EG, f2_fma(gz, gz, f2_fma(gy, gy, f2_mul(gx, gx))));
+                                    F2 gx = f2_sub(upp, cc), gy = f2_sub(ipp, cc), gz = f2_sub(kpp, cc);
+                                    if constexpr (DSUM) {   /* the generic kernel's form */
+                                        gx = f2_mul(gx, P_IA);
+                                        gy = f2_mul(gy, P_IA);
+                                        gz = f2_mul(gz, P_IA);
+                                    }
+                                    eg = f2_mul(DSUM ? P_HALF : P_EG, f2_fma(gz, gz, f2_fma(gy, gy, f2_mul(gx, gx))));
                                     v[S_EG] = eg;
                                 }
                                 if constexpr (SUMS == SUM_FULL) {
@@ -579,6 +600,15 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                             }
     #pragma unroll
                             for (int q = 0; q < NA; ++q) {
+                                if constexpr (DSUM) {
+                                    F2 x = v01[q], y = v23[q];
+                                    if (q >= Q_EK && q <= Q_V) {
+                                        x = f2_mul(x, x);
+                                        y = f2_mul(y, y);
+                                    }
+                                    x = f2_add(x, y);
+                                    dacc[q] = __dadd_rn(dacc[q], (double)(f2_lo(x) + f2_hi(x)));
+                                } else
                                 /* the energies (and the previous half step's kinetic sum, which
                                  * enters the time-centred Ekin) are compensated, per half of the
                                  * pair; the field averages and the sums of squares behind the
@@ -623,12 +653,36 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                             const T lap = A::add(A::add(t0, t1), t2);
                             const T flap = A::mul(fl, lap);
                             const T force =
-                                A::sub(dx2_pow2 ? A::mul(flap, inv_dx2) : A::div(flap, dx2), A::mul(fv, dV<T>(k, cur)));
+                                A::sub(over(flap), A::mul(fv, dV<T>(k, cur)));
                             const T pic = Vec<T>::get(pv, s);
                             const T pn = A::add(pic, A::mul(dt, force));
                             Vec<T>::set(pi_new, s, pn);
                             Vec<T>::set(phi_new, s, DF ? cur : A::add(cur, A::mul(dt, pn)));
-                            if (SUMS != SUM_NONE && (!RAG || s < sites)) {
+                            if constexpr (SUMS == SUM_LINE) {
+                                /* the sums of pi^2, |grad|^2 and their squares; their weights at the
+                                 * item's end (24 operations in double instead of 51 and three divisions:
+                                 * a reporting step of 256^3 195 -> 111 us, expanding 304 -> 137) */
+                                if (!RAG || s < sites) {
+                                    const double gx = A::sub(Vec<T>::get(up, s), cur), gy = A::sub(nxt, cur),
+                                                 gz = A::sub(kpl, cur);
+                                    const double g2 = __fma_rn(gz, gz, __fma_rn(gy, gy, A::mul(gx, gx)));
+                                    const double p2 = A::mul(pn, pn), f2 = A::mul(cur, cur);
+                                    const double ep =
+                                        __fma_rn(f2, __fma_rn(cur, __fma_rn(cur, k.v4, -k.v3), k.v2), k.dv);
+                                    const double et = __fma_rn((double)kin_w, p2, __fma_rn(eg_w, g2, ep));
+                                    dacc[S_V] = A::add(dacc[S_V], pn);
+                                    dacc[S_EK] = A::add(dacc[S_EK], p2);
+                                    dacc[S_EKIN_IN] = __fma_rn(pic, pic, dacc[S_EKIN_IN]);
+                                    dacc[S_PHI] = A::add(dacc[S_PHI], cur);
+                                    dacc[Q_PHI] = A::add(dacc[Q_PHI], f2);
+                                    dacc[S_EP] = A::add(dacc[S_EP], ep);
+                                    dacc[Q_EP] = __fma_rn(ep, ep, dacc[Q_EP]);
+                                    dacc[S_EG] = A::add(dacc[S_EG], g2);
+                                    dacc[Q_EG] = __fma_rn(g2, g2, dacc[Q_EG]);
+                                    dacc[Q_EK] = __fma_rn(p2, p2, dacc[Q_EK]);
+                                    dacc[Q_ET] = __fma_rn(et, et, dacc[Q_ET]);
+                                }
+                            } else if (SUMS != SUM_NONE && (!RAG || s < sites)) {
                                 T eg = (T)0;
                                 if constexpr (want_eg) {
                                     /* forward gradients: x <- axis 1, y <- axis 0, z <- axis 2 (bubble.cpp:794-801) */
@@ -714,7 +768,17 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     #pragma unroll
                     for (int s = 0; s < NS; ++s) {
                         double x = acc[s].value();
-                        if constexpr (std::is_same<T, float>::value)
+                        if constexpr (DSUM) {
+                            x = dacc[s];
+                        } else if constexpr (SUMS == SUM_LINE) {
+                            const double kw = cs->kin_w, vw = cs->vel_w;
+                            x = s == Q_V ? __dmul_rn(__dmul_rn(vw, vw), dacc[S_EK]) : dacc[s];
+                            if (s == S_EK || s == S_EKIN_IN) x = __dmul_rn(kw, x);
+                            if (s == S_V) x = __dmul_rn(vw, x);
+                            if (s == S_EG) x = __dmul_rn(eg_w, x);
+                            if (s == Q_EG) x = __dmul_rn(__dmul_rn(eg_w, eg_w), x);
+                            if (s == Q_EK) x = __dmul_rn(__dmul_rn(kw, kw), x);
+                        } else if constexpr (std::is_same<T, float>::value)
                             x = __dadd_rn(kacc[s].value(), __dadd_rn((double)f2_lo(pacc[s]), (double)f2_hi(pacc[s])));
     #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) x = __dadd_rn(x, __shfl_down_sync(0xffffffffu, x, o));
@@ -805,7 +869,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
         if (is_last && warp < CW) {
             __threadfence();   /* every block's rows are counted: read them after this */
             sum_rows_consumers<NS>(partials, (unsigned)items, ms_tot, item_red[0]);
-            if (warp == 0) epilogue(k, st, ms_tot, !DF, SUMS == SUM_FULL, lane);
+            if (warp == 0) epilogue(k, st, ms_tot, !DF, FULL, lane);
         }
     }
 }
@@ -948,9 +1012,11 @@ cudaError_t launch_step3(int prec, const StepConst &k, bool df, int sums, const 
         if (e != cudaSuccess) return e;                                                                            \
     } while (0)
     if (prec == P_FP64) {
-        if (df && sums == SUM_FULL) CB_LAUNCH3(double, true, SUM_FULL);
+        if (df && sums == SUM_FULL && !k.want_local) CB_LAUNCH3(double, true, SUM_LINE);
+        else if (df && sums == SUM_FULL) CB_LAUNCH3(double, true, SUM_FULL);
         else if (df && k.alpha == 1) CB_LAUNCH3(double, true, SUM_FRIEDMANN_EG);
         else if (df) CB_LAUNCH3(double, true, SUM_FRIEDMANN);
+        else if (sums == SUM_FULL && !k.want_local) CB_LAUNCH3(double, false, SUM_LINE);
         else if (sums == SUM_FULL) CB_LAUNCH3(double, false, SUM_FULL);
         else CB_LAUNCH3(double, false, SUM_NONE);
     } else {

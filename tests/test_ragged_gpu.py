@@ -84,3 +84,23 @@ def test_ragged_start_built_on_the_device(prec):
     most = tol * np.abs(b.phi).max()
     assert np.abs(a.phi - b.phi).max() <= most
     assert np.abs(a.pi - b.pi).max() <= 6 * (0.1 * L / n) * 12 / (L / n) ** 2 * most
+
+
+@pytest.mark.parametrize("n,expansion", [(64, 0), (64, 1), (65, 0), (65, 1)])
+def test_line_without_local_arrays_equals_line_with_them(n, expansion):
+    """The reporting step's sums in double, with and without the local energy
+    arrays (two variants of the staged kernel): each term within a few roundings,
+    N of them added."""
+    import coolbubble_b200 as cb
+    L = n / 10.0   # dx^2 no power of two
+    p = cb.make_params(3, n, L, 4.0, 0.1 * L / n, expansion=expansion, mpl=10.0)
+    start = 0.4 + smooth_noise(3, n, 0.1, seed=5), smooth_noise(3, n, 0.05, seed=6)
+    a, b = cb.Bubble(p, *start), cb.Bubble(p, *start)
+    la, lb = a.step(3, sums=True, local=False), b.step(3, sums=True, local=True)
+    tol = (n ** 3 + 16) * 2.0 ** -53
+    for key in ("etot", "ekin", "egrad", "epot", "etot_var", "ekin_var", "egrad_var", "epot_var", "avphi_var",
+                "avphip_var", "a", "ekin_half_prev"):
+        assert abs(la[key] - lb[key]) <= tol * abs(lb[key]), key
+    for key in ("avphi", "avphip"):
+        assert abs(la[key] - lb[key]) <= tol * (n ** 3 * lb[key + "_var"]) ** 0.5, key
+    np.testing.assert_array_equal(a.phi, b.phi)
