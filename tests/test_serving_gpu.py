@@ -155,3 +155,27 @@ def test_injected_worker_failure_fails_runs_and_refuses_new_ones():
         pool.submit(_params(2, 64, 16.0, 4.0), ic_params(), 10)
     assert "worker stopped" in str(e.value)
     pool.close()
+
+
+@pytest.mark.parametrize("d,n", [(2, 1024), (2, 1447), (3, 160)])
+def test_large_fields_are_delivered_whole(d, n):
+    """Fields of several MiB are taken over in pieces: every site equals the run
+    stepped alone, and the pieces can be collected more than once."""
+    from coolbubble_b200 import _lib as L
+    from coolbubble_b200.serving import DONE, Pool, create_from_seed, ic_params
+    p, ic = _params(d, n, n / 8.0, 4.0), ic_params(1, position_seed=n)
+    with_pool = Pool(8 * 10 ** 9, 2)
+    rid = with_pool.submit(p, ic, 4, sums_every=2, want_fields=True)
+    assert with_pool.wait(rid) == 0
+    first, second = (with_pool.result(rid, n_sites=n ** d) for _ in range(2))
+    with_pool.close()
+    b = create_from_seed(p, ic)
+    lines = [b.step(2), b.step(2)]
+    phi = np.empty(n ** d, np.float32)
+    pi = np.empty(n ** d, np.float32)
+    L.check(L.lib.cb_get_fields_f32(b._h, L.fptr(phi), L.fptr(pi), None, None, None), b._h)
+    b.close()
+    for got in (first, second):
+        assert got["state"] == DONE and [x["etot"] for x in got["lines"]] == [x["etot"] for x in lines]
+        np.testing.assert_array_equal(got["phi"], phi)
+        np.testing.assert_array_equal(got["pi"], pi)
