@@ -5,7 +5,8 @@
  * reported ones needs a global sum). One launch reads phi_n, pi_{n-1/2} and
  * writes phi_{n+2}, pi_{n+3/2}: half the DRAM bytes per step.
  *
- *  - Float and double; rows of a warp or more, padded to whole 16-byte vectors. Tiles of TJ full rows of axis 1 (axis-2 neighbours wrap in shared
+ *  - Float and double; rows of a warp or more, padded to whole 16-byte vectors.
+ *    Tiles of TJ full rows of axis 1, TJ even (axis-2 neighbours wrap in shared
  *    memory; the last tile may hang over the lattice's end and repeat its first
  *    rows); work items (plane part, tile) taken from a device-wide queue,
  *    part-major with tiles fastest (the items in flight share their halo rows
@@ -29,10 +30,13 @@
  *    f32x2, the same rounded operations), so two blocked steps give the fields
  *    of two single steps bit for bit.
  *  - What bounds it: the latency of a round (load, two dependent updates, a
- *    barrier) over 16 warps, ncu on 256^3: float FMA pipe 62 % busy, issue 55 %;
- *    double FP64 pipe 36 %, issue 50 %; DRAM 41-47 %. us per step, one step per
- *    pass -> here: 192^3 float 19.0 -> 16.2, 256^3 50.0 -> 27.3, 512^3 336 ->
- *    193, 256^3 double 89 -> 60, 192^3 double 44.7 -> 28.9.
+ *    barrier) over 16 warps, ncu on 256^3: float FMA pipe 48 % busy (a quarter of
+ *    it register moves), issue 49 %; double FP64 pipe 36 %, issue 50 %; DRAM
+ *    41-47 %. us per step, one step per pass -> here: 192^3 float 19.0 -> 14.7,
+ *    250^3 48 -> 26.2, 256^3 50.0 -> 24.0, 512^3 336 -> 170; double 192^3 44.7 ->
+ *    28.3, 256^3 89 -> 56. A barrier split into arriving and waiting half a round
+ *    later, with two or three level-1 planes, cost more in registers than it hid
+ *    (250^3 30.4 and 34.1, 512^3 184 and 212).
  *  - Waits are bounded (clock64 limit, sleeping retries); a timed-out block
  *    records an error word; consumer warps leave together (a vote in the
  *    per-round barrier).
@@ -67,20 +71,24 @@ constexpr int TB_IQ = 8;
 template <typename T, int BY>
 struct Step;
 
-/* float: packed pairs (f32x2); one site: both halves of a pair carry it (each
- * half is rounded on its own) */
+/* float: packed pairs (f32x2) */
 template <int BY>
 struct Step<float, BY> {
     F2 idx2, dt, nc2, c3, nc4, m2;
     __device__ __forceinline__ explicit Step(const StepConst &k)
         : idx2(f2_splat(k.inv_dx2f)), dt(f2_splat(k.dtf)), nc2(f2_splat(-k.c2f)), c3(f2_splat(k.c3f)),
           nc4(f2_splat(-k.c4f)), m2(f2_splat(-2.f)) {}
-    __device__ __forceinline__ void pair(F2 cc, F2 umm, F2 upp, F2 imm, F2 ipp, F2 kmm, F2 kpp, F2 pp, F2 &phi2,
+    /* the axis-2 term of site c between a and b: in scalars, since the neighbours
+     * of a pair straddle the pairs they are held in (packing them took six moves
+     * per vector) */
+    static __device__ __forceinline__ float along(float a, float c, float b) {
+        return __fadd_rn(__fmaf_rn(c, -2.f, b), a);
+    }
+    __device__ __forceinline__ void pair(F2 cc, F2 umm, F2 upp, F2 imm, F2 ipp, F2 t2, F2 pp, F2 &phi2,
                                          F2 &pi2) const {
         /* x - 2 c in one rounding: 2 c is exact */
         const F2 t0 = f2_add(f2_fma(cc, m2, ipp), imm);
         const F2 t1 = f2_add(f2_fma(cc, m2, upp), umm);
-        const F2 t2 = f2_add(f2_fma(cc, m2, kpp), kmm);
         const F2 lap = f2_add(f2_add(t0, t1), t2);
         /* -V'(f)/f = -(c2 + f (-c3 + f c4)) with every operand negated: the
          * exact negation of the one-step kernel's rounded h (round to nearest
@@ -94,12 +102,11 @@ struct Step<float, BY> {
     __device__ __forceinline__ void operator()(const float4 &c, const float4 &um, const float4 &up, const float4 &im,
                                                const float4 &ip, float left, float right, const float4 &pv,
                                                float4 &phi, float4 &pi) const {
-        const F2 mid = f2_pack(c.y, c.z);
         F2 phi01, pi01, phi23, pi23;
         pair(f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y), f2_pack(ip.x, ip.y),
-             f2_pack(left, c.x), mid, f2_pack(pv.x, pv.y), phi01, pi01);
+             f2_pack(along(left, c.x, c.y), along(c.x, c.y, c.z)), f2_pack(pv.x, pv.y), phi01, pi01);
         pair(f2_pack(c.z, c.w), f2_pack(um.z, um.w), f2_pack(up.z, up.w), f2_pack(im.z, im.w), f2_pack(ip.z, ip.w),
-             mid, f2_pack(c.w, right), f2_pack(pv.z, pv.w), phi23, pi23);
+             f2_pack(along(c.y, c.z, c.w), along(c.z, c.w, right)), f2_pack(pv.z, pv.w), phi23, pi23);
         phi = make_float4(f2_lo(phi01), f2_hi(phi01), f2_lo(phi23), f2_hi(phi23));
         pi = make_float4(f2_lo(pi01), f2_hi(pi01), f2_lo(pi23), f2_hi(pi23));
     }
@@ -108,17 +115,18 @@ struct Step<float, BY> {
                                                float2 &phi, float2 &pi) const {
         F2 p2, q2;
         pair(f2_pack(c.x, c.y), f2_pack(um.x, um.y), f2_pack(up.x, up.y), f2_pack(im.x, im.y), f2_pack(ip.x, ip.y),
-             f2_pack(left, c.x), f2_pack(c.y, right), f2_pack(pv.x, pv.y), p2, q2);
+             f2_pack(along(left, c.x, c.y), along(c.x, c.y, right)), f2_pack(pv.x, pv.y), p2, q2);
         phi = make_float2(f2_lo(p2), f2_hi(p2));
         pi = make_float2(f2_lo(q2), f2_hi(q2));
     }
+    /* one site: the same operations in scalars */
     __device__ __forceinline__ void operator()(float c, float um, float up, float im, float ip, float left,
                                                float right, float pv, float &phi, float &pi) const {
-        F2 p2, q2;
-        pair(f2_splat(c), f2_splat(um), f2_splat(up), f2_splat(im), f2_splat(ip), f2_splat(left), f2_splat(right),
-             f2_splat(pv), p2, q2);
-        phi = f2_lo(p2);
-        pi = f2_lo(q2);
+        const float lap = __fadd_rn(__fadd_rn(along(im, c, ip), along(um, c, up)), along(left, c, right));
+        const float nh = __fmaf_rn(c, __fmaf_rn(c, f2_lo(nc4), f2_lo(c3)), f2_lo(nc2));
+        const float force = __fmaf_rn(lap, f2_lo(idx2), __fmul_rn(c, nh));
+        pi = __fmaf_rn(f2_lo(dt), force, pv);
+        phi = __fmaf_rn(f2_lo(dt), pi, c);
     }
 };
 
@@ -152,17 +160,18 @@ struct Step<double, BY> {
  * with its columns along axis 0 kept in registers:
  *   x_m, x_c  input phi at planes m - 1, m (level 1 at plane m reads phi at
  *             m + 1 from the stage that just landed);
- *   y_m, y_c, y_p  level-1 phi at planes m' - 1, m', m' + 1 (level 2 at m');
+ *   y_c, y_p  level-1 phi at planes m', m' + 1 (level 2 at m');
  *   z, zz     level-1 pi at planes m', m' + 1.
  * The halo rows (j0 - 1, j0 + tj) are updated at level 1 only; a thread's
  * share of them keeps only x_m, x_c. */
 template <typename V>
 struct Slot {
-    V x_m, x_c, y_m, y_c, y_p, z, zz;
+    V x_m, x_c, y_c, y_p, z, zz;
 };
 
 /* Two leapfrog steps per pass (see the file comment). Thread c owns the tile
- * positions c and NT + c (NT = tile positions / 2 = threads) and HW sites of
+ * positions c and c + half the tile's (the same site of the row half a tile
+ * further, so one set of offsets and row ends serves both) and HW sites of
  * the halo rows (row j0 - 1, then row j0 + tj), sites HW c .. HW c + HW - 1:
  * HW = 2 n / NT (1 or 2) gives every thread the same share; HW = 4 gives
  * threads c < 2 n / 4 one vector each (where 2 n / NT is not 1 or 2). Rows hold a
@@ -172,7 +181,8 @@ struct Slot {
  * branch on the halo slot is uniform across the warp.
  * NV: the vectors of a row where they are a power of two (32, 64, 128) and the
  * tile has 1024 of them: every shared offset of a round is then a constant
- * (512^3 float 193 -> 177 us per step, 256^3 27.4 -> 24.9, in double 60 -> 55).
+ * (512^3 float 193 -> 177 us per step, 256^3 27.4 -> 24.9, in double 60 -> 55;
+ * with the axis-2 terms in scalars 170 and 24.0).
  * The streamed input planes are counted g = 0, 1, ... over all the block's
  * items (plane g in stage g mod nstage); round g waits for plane g. An item
  * computing planes [p0, p1) streams planes p0 - 2 .. p1 + 1: its first two
@@ -188,6 +198,10 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     using V = typename Vec<T>::V;
     constexpr int W = Vec<T>::W;
     constexpr uint32_t ES = sizeof(T);
+    /* level-1 phi at plane m' - 1 from registers only where offsets are constants:
+     * elsewhere they are too few and keeping it costs more than reading it back (250^3 float 27.7 -> 26.3 us per step,
+     * 192^3 15.6 -> 14.7; 512^3, NV, 170 -> 174) */
+    constexpr bool KEEP_Y = NV != 0;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ int abort_flag;
     __shared__ int item_q[TB_IQ];
@@ -227,7 +241,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * its start up to the lattice's last row, then the rest from row 0 */
     __shared__ size_t pr_r[2];   /* thread 0's only: kept out of the registers */
     __shared__ int pr_c[2];
-    long long issued = 0;                                        /* planes issued so far */
+    int issued = 0;                                              /* planes issued so far */
     int is_stage = 0;                                            /* its stage: issued mod nstage */
     bool pr_done = false;
     auto next_item = [&]() {
@@ -252,7 +266,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         pr_c[0] = min(R0, n - r0);
         pr_c[1] = min(R0p, n - r1);
     };
-    auto issue_upto = [&](long long last) {
+    auto issue_upto = [&](int last) {
         while (!pr_done && issued <= last) {
             const int s = is_stage;
             const int pw = pr_pl < 0 ? pr_pl + n : (pr_pl >= n ? pr_pl - n : pr_pl);
@@ -290,18 +304,12 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     const Step<T, BY> step(k);
     /* the positions as offsets r1 np + kk in an array of level-1 rows (row r1,
      * first site kk; rows hold np = W nvr elements, so tile position u sits at
-     * np + W u): tile slot s at off0 + s W NT, the halo slot at offh. Where the
-     * tile's positions are no multiple of the threads (!WHOLE), the spare ones
-     * repeat the last position and store nothing. */
-    const int npos = tj * (np / W), slot_step = W * NT;
-    int offs[TB_NTS];
-    bool own[TB_NTS];
-#pragma unroll
-    for (int s = 0; s < TB_NTS; ++s) {
-        const int u = threadIdx.x + s * NT;
-        own[s] = WHOLE || u < npos;
-        offs[s] = np + W * (own[s] ? u : npos - 1);
-    }
+     * np + W u): tile slot s, which is half a tile's rows, at off0 + s tj / 2 np,
+     * the halo slot at offh. Where a slot's positions are fewer than the threads
+     * (!WHOLE), the spare threads repeat the last position and store nothing. */
+    const int npos = tj / TB_NTS * (np / W), slot_step = WHOLE ? W * NT : W * npos;
+    const bool own = WHOLE || (int)threadIdx.x < npos;
+    const int off0 = np + W * (own ? (int)threadIdx.x : npos - 1);
     using HT = typename Part<T, HW>::V;
     /* whole warps take part in the halo rows (they shuffle) */
     const bool has_h = HW * (int)(WHOLE ? threadIdx.x : threadIdx.x & ~31) < 2 * np;
@@ -311,28 +319,20 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     /* the axis-2 neighbours of the vector at shared byte address a: from the
      * neighbouring lanes, at the warp's ends and the row's ends from the row
      * (periodic; a row's pad holds the images of its first sites, which advance
-     * as those do). WHOLE: every slot of a thread starts at the same site of its
-     * row (the slots are whole rows apart) and a row is whole warps. */
-    uint32_t from_l[TB_NTS], from_r[TB_NTS];
-    int ladj_b[TB_NTS], radj_b[TB_NTS];
-#pragma unroll
-    for (int s = 0; s < TB_NTS; ++s) {
-        const int kk = offs[s] % np;
-        from_l[s] = lane == 0 || (!WHOLE && kk == 0);
-        from_r[s] = lane == 31 || (!WHOLE && kk + W == np);
-        ladj_b[s] = (int)ES * ((kk == 0 ? n : 0) - 1);
-        radj_b[s] = (int)ES * ((kk + W == np ? -n : 0) + W);
-    }
+     * as those do). Both slots of a thread start at the same site of their rows
+     * (they are whole rows apart). WHOLE: a row is whole warps. */
+    const int kk0 = off0 % np;
+    const uint32_t from_l = lane == 0 || (!WHOLE && kk0 == 0), from_r = lane == 31 || (!WHOLE && kk0 + W == np);
+    const int ladj_b = (int)ES * ((kk0 == 0 ? n : 0) - 1), radj_b = (int)ES * ((kk0 + W == np ? -n : 0) + W);
     /* the same for the halo share (first site kk_h of its row, HW sites) */
     const int kk_h = fh % np;
     const uint32_t from_lh = lane == 0 || (!WHOLE && kk_h == 0), from_rh = lane == 31 || (!WHOLE && kk_h + HW == np);
     const int ladjh_b = (int)ES * ((kk_h == 0 ? n : 0) - 1), radjh_b = (int)ES * ((kk_h + HW == np ? -n : 0) + HW);
-    auto sides = [&](const V &c, uint32_t a, int s, T &left, T &right) {
-        const int q = WHOLE ? 0 : s;
+    auto sides = [&](const V &c, uint32_t a, T &left, T &right) {
         left = __shfl_up_sync(0xffffffffu, last(c), 1);
         right = __shfl_down_sync(0xffffffffu, first(c), 1);
-        lds_if(left, a + ladj_b[q], from_l[q]);
-        lds_if(right, a + radj_b[q], from_r[q]);
+        lds_if(left, a + ladj_b, from_l);
+        lds_if(right, a + radj_b, from_r);
     };
     const uint32_t ring_a = smem_u32(ring), l1_a = smem_u32(l1);
     const uint32_t stage_b = ES * (uint32_t)stage_n, slot_b = ES * (uint32_t)slot_n, nb = ES * (uint32_t)np;
@@ -356,15 +356,15 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     /* end of round g: every thread's reads of the planes and level-1 slots are
      * done and its level-1 writes visible; thread 0 then issues the planes
      * whose stages that freed. Returns whether any thread's wait ran out. */
-    auto end_round = [&](long long g, bool bad) -> bool {
+    auto end_round = [&](int g, bool bad) -> bool {
         const bool any_bad = tb_any(bad);
         if (!any_bad && threadIdx.x == 0) issue_upto(g + nstage - 1);
         return any_bad;
     };
     Slot<V> sl[TB_NTS];
     HT hxm, hxc;
-    auto at = [&](int s) { return WHOLE ? offs[0] + s * slot_step : offs[s]; };
-    long long g = 0;     /* the round: index of the input plane it waits for */
+    auto at = [&](int s) { return off0 + s * slot_step; };
+    int g = 0;     /* the round: index of the input plane it waits for */
     bool bad = false;
     for (int j = 0;; ++j) {
         const int it = item_q[j % TB_IQ];
@@ -375,7 +375,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         /* the slots whose level-2 row is the lattice's (the last tile may hang over) */
         bool keep[TB_NTS];
 #pragma unroll
-        for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own[s] && j0 * np + offs[s] - np < n * np);
+        for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own && j0 * np + at(s) - np < n * np);
         /* input planes p0 - 2 and p0 - 1: this thread's phi into the register queues */
         if (!bad && acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                 const uint32_t S0 = ring_a + gs_prev * stage_b;   /* plane q - 1 */
                 const uint32_t D1 = l1_a + ((q - p0) & 1) * slot_b;   /* level-1 plane q - 1 */
                 /* level 1 at plane q - 1, at one position with input queue (xm, xc) */
-                auto level1 = [&](V &xm, V &xc, int s, V &phi1, V &pi1) {
+                auto level1 = [&](V &xm, V &xc, int s, V &ym, V &phi1, V &pi1) {
                     /* input phi row 0 is level-1 row -1: the centre sits at n + off */
                     const uint32_t ob = ES * (uint32_t)at(s);
                     const V x_p = lds<V>(Sn + nb + ob);
@@ -417,9 +417,11 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                     const V up = lds<V>(S0 + 2u * nb + ob);
                     const V pv = lds<V>(S0 + pi_b + ob);
                     T left, right;
-                    sides(xc, S0 + nb + ob, s, left, right);
+                    sides(xc, S0 + nb + ob, left, right);
                     step(xc, um, up, xm, x_p, left, right, pv, phi1, pi1);
-                    if (own[s]) sts(D1 + ob, phi1);
+                    /* the slot still holds this position's level-1 plane q - 3 */
+                    if (!KEEP_Y) ym = lds<V>(D1 + ob);
+                    if (own) sts(D1 + ob, phi1);
                     xm = xc;
                     xc = x_p;
                 };
@@ -429,14 +431,14 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                 const uint32_t L0 = l1_a + ((m2 - p0 + 1) & 1) * slot_b;
                 /* global row j0 - 1 + r1 of plane m2: the tile position's offset from row j0 - 1 */
                 const size_t gbase = ((size_t)m2 * n + (size_t)j0) * np - (size_t)np;
-                auto level2 = [&](Slot<V> &x, int s) {
+                auto level2 = [&](Slot<V> &x, const V &ym, int s) {
                     const uint32_t ob = L0 + ES * (uint32_t)at(s);
                     const V um = lds<V>(ob - nb);
                     const V up = lds<V>(ob + nb);
                     T left, right;
-                    sides(x.y_c, ob, s, left, right);
+                    sides(x.y_c, ob, left, right);
                     V phi2, pi2;
-                    step(x.y_c, um, up, x.y_m, x.y_p, left, right, x.z, phi2, pi2);
+                    step(x.y_c, um, up, ym, x.y_p, left, right, x.z, phi2, pi2);
                     if (keep[s]) {
                         *reinterpret_cast<V *>(phi_out + (gbase + at(s))) = phi2;
                         *reinterpret_cast<V *>(pi_out + (gbase + at(s))) = pi2;
@@ -447,14 +449,14 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
 #pragma unroll
                 for (int s = 0; s < TB_NTS; ++s) {
                     Slot<V> &x = sl[s];
-                    V phi1, pi1;
-                    level1(x.x_m, x.x_c, s, phi1, pi1);
-                    x.y_m = x.y_c;
+                    V ym, phi1, pi1;
+                    level1(x.x_m, x.x_c, s, ym, phi1, pi1);
+                    if (KEEP_Y) ym = x.y_c;
                     x.y_c = x.y_p;
                     x.y_p = phi1;
                     x.z = x.zz;
                     x.zz = pi1;
-                    if (m2 >= p0) level2(x, s);
+                    if (m2 >= p0) level2(x, ym, s);
                 }
                 if (has_h) {
                     /* level 1 at plane q - 1 on the halo share */
@@ -498,8 +500,8 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         /* record, then let every issued copy land before the block exits */
         if (threadIdx.x == 0) {
             atomicExch(&st->err, ERR_TMA_TIMEOUT);
-            for (long long q = issued > nstage ? issued - nstage : 0; q < issued; ++q)
-                mbar_wait(&full[(int)(q % nstage)], (uint32_t)((q / nstage) & 1), WAIT_LIMIT / 8);
+            for (int q = max(issued - nstage, 0); q < issued; ++q)
+                mbar_wait(&full[q % nstage], (uint32_t)((q / nstage) & 1), WAIT_LIMIT / 8);
         }
         __syncthreads();
     }
@@ -534,7 +536,7 @@ bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage
     const int nv = np / W;
     const long long slots = sm_count();
     double best = 0.0;
-    for (int t = 4; t <= 32 && t * nv <= TB_NTS * TB_MAXT; ++t) {
+    for (int t = 4; t <= 32 && t * nv <= TB_NTS * TB_MAXT; t += TB_NTS) {
         const size_t stage = (size_t)(2 * t + 6) * row, lev = (size_t)2 * (t + 2) * row;
         if (lev + 4 * stage > budget) break;
         const long long ntiles = (n + t - 1) / t;
