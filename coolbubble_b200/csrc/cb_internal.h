@@ -137,6 +137,7 @@ size_t step_blocks(const StepConst &k);
 constexpr size_t STEP2_MIN_SITES = size_t(1) << 20;   /* below 1024^2 both are launch-bound; the tiles win at 128^2 */
 constexpr size_t STEP1_MIN_SITES = size_t(1) << 20;   /* d = 1: at 2^18 sites the tiles still win (4.5 vs 5.7 us) */
 bool step2_applies(const StepConst &k, int prec, bool drift_first);
+bool step2_one_strip(const StepConst &k, int prec);   /* and a row is one block's strip */
 size_t step2_blocks(const StepConst &k);
 cudaError_t launch_step2(int prec, const StepConst &k, int sums, const void *phi_in, const void *pi_in,
                          void *phi_out, void *pi_out, void *le, void *lg, void *lp, DevState *st, double *partials,

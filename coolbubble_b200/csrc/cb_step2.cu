@@ -196,6 +196,13 @@ bool step2_applies(const StepConst &k, int prec, bool drift_first) {
     return k.d == 2 && (size_t)k.n * k.n >= STEP2_MIN_SITES;
 }
 
+bool step2_one_strip(const StepConst &k, int prec) {
+    unsigned strips, bands;
+    int rpb;
+    step2_grid(k, prec, strips, bands, rpb);
+    return step2_applies(k, prec, false) && strips == 1;
+}
+
 size_t step2_blocks(const StepConst &k) {
     size_t b = 0;
     for (int prec = 0; prec < 2; ++prec) {

@@ -637,6 +637,12 @@ int step2tb_steps(const StepConst &k, int prec, int left, bool sums) {
         const int launches = (left + most - 1) / most;
         return (left + launches - 1) / launches;
     }
+    /* The start and the block-wide sums of a launch here are not earned back by the one
+     * step of a small lattice (in us, double: 64^2 9.0, one-step kernel 7.7; 256^2 10.5
+     * and 9.5; 320^2 11.2 and 11.3; 512^2 13.9 and 18.0), by two of a very small one
+     * (32^2 8.8 and 8.6; 64^2 9.4 and 9.3), nor where the strips' kernel has one per row
+     * (1024^2 float 17.0 and 13.7; with two, in double, 21.0 and 22.1). */
+    if (sums && ((left == 1 && (k.n <= 288 || step2_one_strip(k, prec))) || (left == 2 && k.n <= 64))) return 0;
     return even_split(left, [&](int t) {
         Plan2 p;
         return plan_2d(k, prec, t, p) ? p.us : 0.0;

@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     const int items = ntiles * parts;
     const size_t row_bytes = (size_t)np * sizeof(T);
     const size_t plane = (size_t)n * np;
+    const uint32_t tx_bytes = (uint32_t)(((size_t)(tj + 2) + g.pi_rows()) * row_bytes);
     /* rows of the tile from row j0 (RAG: the last one may be short) */
     auto rows_at = [&](int j0) { return RAG ? min(tj, n - j0) : tj; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             const T *src_phi = fphi[sb] + (size_t)pw * plane;
             const T *src_pi = fpi[sb] + (size_t)pw * plane;
             fence_proxy_async();
-            mbar_arrive_expect_tx(&full[s], (uint32_t)((2 * tr + (DF ? 4 : 2)) * row_bytes));
+            mbar_arrive_expect_tx(&full[s], RAG ? (uint32_t)((2 * tr + (DF ? 4 : 2)) * row_bytes) : tx_bytes);
             bulk_g2s(dst + np, src_phi + (size_t)j0 * np, (uint32_t)(tr * row_bytes), &full[s]);
             bulk_g2s(dst, src_phi + (size_t)jm * np, (uint32_t)row_bytes, &full[s]);
             bulk_g2s(dst + (size_t)(tr + 1) * np, src_phi + (size_t)jp * np, (uint32_t)row_bytes, &full[s]);
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                 }
                 int t, p0, p1;
                 item_of(it, t, p0, p1);
-                const int j0 = t * tj, nvec = rows_at(j0) * nvec_row, nv_drift = nvec + 2 * nvec_row;
+                const int j0 = t * tj, nvec = RAG ? rows_at(j0) * nvec_row : tj * nvec_row, nv_drift = nvec + 2 * nvec_row;
                 if (SUMS != SUM_NONE) {
     #pragma unroll
                     for (int s = 0; s < NSUM; ++s) {
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                         const VT ip = *reinterpret_cast<const VT *>(Sp + c_off);
                         const VT pv = *reinterpret_cast<const VT *>(P0 + r * np + kk);
                         const int lo = (r + 1) * np + (kk == 0 ? n - 1 : kk - 1);
-                        const int ro = (r + 1) * np + (kk + W >= n ? kk + W - n : kk + W);
+                        const int ro = (r + 1) * np + (RAG ? (kk + W >= n ? kk + W - n : kk + W) : (kk + W == n ? 0 : kk + W));
                         const T left = S0[lo];
                         const T right = S0[ro];
                         /* RAG: the row's last vector holds `sites` sites, then images of the

@@ -15,6 +15,7 @@ POSITIVE = ("etot", "ekin", "egrad", "epot", "etot_var", "ekin_var", "egrad_var"
     (2, 16, 2.0), (2, 32, 3.2), (2, 128, 16.0),   # a whole row on 8, 16 or 32 lanes
     (2, 64, 8.0), (2, 101, 12.625), (2, 250, 25.0),   # vectors, odd rows (site by site), double vectors only
     (2, 512, 32.0), (2, 1000, 100.0), (2, 1031, 103.1),   # several tiles, tiles over the end, more tiles than blocks
+    (2, 288, 28.8), (2, 1024, 102.4),   # single steps with sums: the one-step kernels (1024: one strip a row)
     (2, 502, 30.0),       # dx^2 has no two-operation division: the compiler's divides
     (1, 3, 0.3), (1, 130, 16.25), (1, 4097, 409.7), (1, 1 << 18, 26214.4)])
 @pytest.mark.parametrize("prec", ["fp64", "fp32c"])
