@@ -169,7 +169,7 @@ StepConst make_const(const cb_params *p) {
     k.want_local = 0;
     const char *path = std::getenv("CB_STEP_PATH");
     k.force_generic = (path && std::string(path) == "generic") ? 1 : 0;
-    /* steps per pass of the static float 3-D step: CB_TEMPORAL_BLOCK=1 or 2 fixes it;
+    /* steps per pass of the static 3-D step: CB_TEMPORAL_BLOCK=1 or 2 fixes it;
      * unset, it is chosen per lattice size by timing both passes once (0: not chosen yet) */
     const char *tb = std::getenv("CB_TEMPORAL_BLOCK");
     k.temporal = tb ? std::max(1, std::atoi(tb)) : 0;

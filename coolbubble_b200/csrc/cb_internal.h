@@ -82,7 +82,7 @@ struct StepConst {
     int alpha, expanding;
     int want_local;
     int force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
-    int temporal;       /* steps per pass for static float 3-D lattices (1: no temporal blocking) */
+    int temporal;       /* steps per pass for static 3-D lattices (1: no temporal blocking) */
     /* fields below: behind those that the kernels load in groups of 16 bytes */
     int pitch;          /* elements from a row of the last axis to the next: n, or (d = 3 runs) n rounded
                            up to whole 16-byte vectors. The pad holds the periodic images of the row's
@@ -183,7 +183,7 @@ cudaError_t launch_step3_df(int prec, const StepConst &k, int nsteps, bool coope
 bool step3df_applies(const StepConst &k, int prec);
 size_t step3df_partial_rows(const StepConst &k, int prec);
 
-/* TL steps per pass, static float 3-D lattices (cb_step3_tb.cu). */
+/* TL steps per pass, static 3-D lattices (cb_step3_tb.cu). */
 bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage, size_t &smem, unsigned &grid,
                       int &parts);
 cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *phi_in, const void *pi_in,

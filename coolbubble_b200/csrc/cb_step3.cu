@@ -21,7 +21,7 @@
  *    (RAG) whose pad repeats the row's first sites; the images advance with the
  *    same vector operations as the sites and take no part in the sums. 250^3 in
  *    float, which the generic kernel took site by site at 88 us per step, runs at
- *    48 here and 29.7 in two-step passes (256^3: 50 and 28).
+ *    48 here and 26.2 in two-step passes (256^3: 50 and 24.0).
  *  - Each thread updates 16-byte vectors (4 floats / 2 doubles) and stores
  *    phi and pi with 128-bit coalesced writes.
  *  - Drift-first (expanding background): the pending drift of the previous
@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             };
             auto grad = [&](T dphi) -> T { return adx_pow2 ? A::mul(dphi, inv_adx) : A::div(dphi, adx); };
             const int nvec_row = np / W;
+            const int nvec_all = tj * nvec_row, nv_drift_all = (tj + 2) * np / W;   /* !RAG: of every tile */
             const int row_step = NC / nvec_row, vec_step = NC % nvec_row;
             constexpr bool want_eg = FULL || SUMS == SUM_FRIEDMANN_EG;
             /* float steps run in packed f32x2 pairs, with or without sums */
@@ -457,7 +458,8 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                 }
                 int t, p0, p1;
                 item_of(it, t, p0, p1);
-                const int j0 = t * tj, nvec = RAG ? rows_at(j0) * nvec_row : tj * nvec_row, nv_drift = nvec + 2 * nvec_row;
+                const int j0 = t * tj;
+                const int nvec = RAG ? rows_at(j0) * nvec_row : nvec_all, nv_drift = RAG ? nvec + 2 * nvec_row : nv_drift_all;
                 if (SUMS != SUM_NONE) {
     #pragma unroll
                     for (int s = 0; s < NSUM; ++s) {

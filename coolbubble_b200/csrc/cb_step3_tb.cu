@@ -202,6 +202,10 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * elsewhere they are too few and keeping it costs more than reading it back (250^3 float 27.7 -> 26.3 us per step,
      * 192^3 15.6 -> 14.7; 512^3, NV, 170 -> 174) */
     constexpr bool KEEP_Y = NV != 0;
+    /* 64 bits for the registers the compiler then assigns: 256^3 double 56.2 -> 55.3 us
+     * per step, while the general rows are faster with 32 (250^3 float 28.3 -> 27.7,
+     * double 61.2 -> 60.4) */
+    using Count = std::conditional_t<NV != 0 && std::is_same<T, double>::value, long long, int>;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ int abort_flag;
     __shared__ int item_q[TB_IQ];
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * its start up to the lattice's last row, then the rest from row 0 */
     __shared__ size_t pr_r[2];   /* thread 0's only: kept out of the registers */
     __shared__ int pr_c[2];
-    int issued = 0;                                              /* planes issued so far */
+    Count issued = 0;                                            /* planes issued so far */
     int is_stage = 0;                                            /* its stage: issued mod nstage */
     bool pr_done = false;
     auto next_item = [&]() {
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         pr_c[0] = min(R0, n - r0);
         pr_c[1] = min(R0p, n - r1);
     };
-    auto issue_upto = [&](int last) {
+    auto issue_upto = [&](Count last) {
         while (!pr_done && issued <= last) {
             const int s = is_stage;
             const int pw = pr_pl < 0 ? pr_pl + n : (pr_pl >= n ? pr_pl - n : pr_pl);
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     /* end of round g: every thread's reads of the planes and level-1 slots are
      * done and its level-1 writes visible; thread 0 then issues the planes
      * whose stages that freed. Returns whether any thread's wait ran out. */
-    auto end_round = [&](int g, bool bad) -> bool {
+    auto end_round = [&](Count g, bool bad) -> bool {
         const bool any_bad = tb_any(bad);
         if (!any_bad && threadIdx.x == 0) issue_upto(g + nstage - 1);
         return any_bad;
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     Slot<V> sl[TB_NTS];
     HT hxm, hxc;
     auto at = [&](int s) { return off0 + s * slot_step; };
-    int g = 0;     /* the round: index of the input plane it waits for */
+    Count g = 0;   /* the round: index of the input plane it waits for */
     bool bad = false;
     for (int j = 0;; ++j) {
         const int it = item_q[j % TB_IQ];
@@ -500,7 +504,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         /* record, then let every issued copy land before the block exits */
         if (threadIdx.x == 0) {
             atomicExch(&st->err, ERR_TMA_TIMEOUT);
-            for (int q = max(issued - nstage, 0); q < issued; ++q)
+            for (int q = max((int)issued - nstage, 0); q < (int)issued; ++q)
                 mbar_wait(&full[q % nstage], (uint32_t)((q / nstage) & 1), WAIT_LIMIT / 8);
         }
         __syncthreads();
