@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             const double eg_w = SUMS == SUM_LINE ? __ddiv_rn(0.5, __dmul_rn(cs->adx, cs->adx)) : 0.0;
             /* wait for the ring position under cursor c to land */
             auto acquire = [&](const Cursor &c) -> bool {
-                const bool ok = abort_flag == 0 && mbar_wait(&full[c.s], c.ph, WAIT_LIMIT);
+                const bool ok = warp_all(abort_flag == 0 && mbar_wait(&full[c.s], c.ph, WAIT_LIMIT));
                 if (!ok) atomicExch(&abort_flag, 1);
                 return ok;
             };
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
             };
             /* wait until every consumer thread drifted its share of the plane under c */
             auto drifted_wait = [&](const Cursor &c) -> bool {
-                const bool ok = abort_flag == 0 && mbar_wait(&drifted[c.s], c.ph, WAIT_LIMIT);
+                const bool ok = warp_all(abort_flag == 0 && mbar_wait(&drifted[c.s], c.ph, WAIT_LIMIT));
                 if (!ok) atomicExch(&abort_flag, 1);
                 return ok;
             };
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
              * consumer warp then takes the same exit (a vote in the barrier) when a
              * wait runs out */
             for (; run; ++j) {
-                if (abort_flag != 0 || !mbar_wait(&item_full[j % IQ], (uint32_t)((j / IQ) & 1), WAIT_LIMIT)) {
+                if (!warp_all(abort_flag == 0 && mbar_wait(&item_full[j % IQ], (uint32_t)((j / IQ) & 1), WAIT_LIMIT))) {
                     atomicExch(&abort_flag, 1);
                     run = false;
                 }

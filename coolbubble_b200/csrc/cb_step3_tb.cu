@@ -351,11 +351,21 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
             gph ^= 1u;
         }
     };
-    /* round g: wait for input plane g; false (and the abort flag) if the wait ran out */
+    /* Round g: wait for input plane g; a wait that ran out sets the abort flag and
+     * bad, which the vote at the round's end makes the block's. The round's shuffles
+     * need every lane of a warp whatever its own wait gave, so in float the round
+     * runs in any case (what it stores belongs to a step reported as failed); in
+     * double, where the registers come out better for it, whole warps skip it.
+     * us per step with the skip and without, float: 192^3 14.9 and 14.2, 250^3 26.4
+     * and 25.5, 512^3 172 and 172; double: 192^3 28.7 and 27.2, 250^3 61.1 and 63.4,
+     * 256^3 56.4 and 56.6. */
+    constexpr bool SKIP = std::is_same<T, double>::value;
+    bool bad = false;
     auto acquire = [&]() -> bool {
-        const bool ok = mbar_wait(&full[gs], gph, WAIT_LIMIT);   /* a wait that ran out is voted on below */
+        const bool ok = mbar_wait(&full[gs], gph, WAIT_LIMIT);
         if (!ok) atomicExch(&abort_flag, 1);
-        return ok;
+        bad = !ok;
+        return !SKIP || warp_all(ok);
     };
     /* end of round g: every thread's reads of the planes and level-1 slots are
      * done and its level-1 writes visible; thread 0 then issues the planes
@@ -369,7 +379,6 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     HT hxm, hxc;
     auto at = [&](int s) { return off0 + s * slot_step; };
     Count g = 0;   /* the round: index of the input plane it waits for */
-    bool bad = false;
     for (int j = 0;; ++j) {
         const int it = item_q[j % TB_IQ];
         if (it < 0) break;
@@ -381,24 +390,20 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
 #pragma unroll
         for (int s = 0; s < TB_NTS; ++s) keep[s] = WHOLE || (own && j0 * np + at(s) - np < n * np);
         /* input planes p0 - 2 and p0 - 1: this thread's phi into the register queues */
-        if (!bad && acquire()) {
+        if (acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
 #pragma unroll
             for (int s = 0; s < TB_NTS; ++s) sl[s].x_m = lds<V>(S + ES * at(s));
             if (has_h) hxm = lds<HT>(S + ES * offh);
-        } else {
-            bad = true;
         }
         if (end_round(g, bad)) break;
         ++g;
         advance();
-        if (!bad && acquire()) {
+        if (acquire()) {
             const uint32_t S = ring_a + gs * stage_b + nb;
 #pragma unroll
             for (int s = 0; s < TB_NTS; ++s) sl[s].x_c = lds<V>(S + ES * at(s));
             if (has_h) hxc = lds<HT>(S + ES * offh);
-        } else {
-            bad = true;
         }
         if (end_round(g, bad)) break;
         ++g;
@@ -408,7 +413,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
          * 0.2225 ms per step; no spills at 128 registers) */
 #pragma unroll 2
         for (int q = p0; q <= p1 + 1; ++q, ++g, advance()) {
-            if (!bad && acquire()) {
+            if (acquire()) {
                 const uint32_t Sn = ring_a + gs * stage_b;        /* plane q */
                 const uint32_t S0 = ring_a + gs_prev * stage_b;   /* plane q - 1 */
                 const uint32_t D1 = l1_a + ((q - p0) & 1) * slot_b;   /* level-1 plane q - 1 */
@@ -480,8 +485,6 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
                     hxm = hxc;
                     hxc = xp;
                 }
-            } else {
-                bad = true;
             }
             if (end_round(g, bad)) {
                 bad = true;

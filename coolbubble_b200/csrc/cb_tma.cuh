@@ -61,6 +61,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
     return true;
 }
 
+/* One answer for all lanes of a warp: a bounded wait that ran out in some of
+ * them only (a lane gives up by its own clock) has run out, since the shuffles
+ * and warp barriers that follow need every lane. Every lane calls it. */
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
