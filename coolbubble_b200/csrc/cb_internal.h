@@ -89,9 +89,11 @@ struct StepConst {
                            first sites: every kernel that writes phi or pi keeps them equal */
     int odd;            /* the step's index is odd: expanding steps march the planes in turn forwards and
                            backwards */
-    int dx2_pair;       /* fma(x, inv_dx2, x inv_dx2_lo) is x / dx2 rounded (reciprocal_pair, cb_api.cpp) */
-    double inv_dx2_lo;  /* 1/dx2 - inv_dx2, rounded */
+    int dx2_pair;       /* fma(x, inv_dx2_hi, x inv_dx2_lo) is x / dx2 rounded */
+    double inv_dx2_hi, inv_dx2_lo;   /* 1/dx2 as a pair (reciprocal_pair, cb_api.cpp) */
 };
+
+bool reciprocal_pair(double d, double &zh, double &zl);
 
 /* The checks of one line from its energies, in double and in this order (the
  * step epilogue does the same operations with explicit rounding):
