@@ -175,11 +175,10 @@ StepConst make_const(const cb_params *p) {
     k.dx2 = k.dx * k.dx;
     k.inv_dx2 = 1.0 / k.dx2;
     k.dx2_pow2 = is_pow2_host(k.dx2);
-    k.dx2_pair = reciprocal_pair(k.dx2, k.inv_dx2_hi, k.inv_dx2_lo);
-    k.dtf = (float)k.dt;
-    k.dxf = (float)k.dx;
-    k.dx2f = (float)k.dx2;
     k.inv_dx2f = (float)k.inv_dx2;
+    k.dx2_pair = reciprocal_pair(k.dx2, k.inv_dx2, k.inv_dx2_lo);
+    k.dtf = (float)k.dt;
+    k.dx2f = (float)k.dx2;
     k.dxLD = std::pow(k.dx / p->L, p->d);       /* bubble.hpp:47 */
     k.mpl = p->mpl;
     k.alpha = p->alpha;
@@ -190,7 +189,7 @@ StepConst make_const(const cb_params *p) {
     /* steps per pass of the static 3-D step: CB_TEMPORAL_BLOCK=1 or 2 fixes it;
      * unset, it is chosen per lattice size by timing both passes once (0: not chosen yet) */
     const char *tb = std::getenv("CB_TEMPORAL_BLOCK");
-    k.temporal = tb ? std::max(1, std::atoi(tb)) : 0;
+    k.temporal = (short)(tb ? std::min(std::max(1, std::atoi(tb)), 99) : 0);
     if (k.force_generic) k.temporal = 1;
     return k;
 }
@@ -572,7 +571,7 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
     int tj, ns, parts;
     size_t sm;
     unsigned g;
-    if (h->p.d == 3 && h->k.temporal == 0 && nsteps > 2) h->k.temporal = choose_temporal(h);
+    if (h->p.d == 3 && h->k.temporal == 0 && nsteps > 2) h->k.temporal = (short)choose_temporal(h);
     const int tl = h->k.temporal;
     const bool tb_ok = !h->expanding && h->unit_scale && tl > 1 &&
                        step3tb_geometry(h->k, h->prec, tl, tj, ns, sm, g, parts);

@@ -64,7 +64,12 @@ struct DevState {
     unsigned int pad1;
 };
 
-/* Constants of one run, passed by value to every launch. */
+/* Constants of one run, passed by value to every launch.
+ * Its size decides what a launch costs the host: with the bytes of all arguments
+ * at 24 or 32 beyond a multiple of 64 a launch takes 1.9 us, else 2.2 to 2.3
+ * (216 to 416 bytes tried, every 8). The 1-D and 2-D kernels, whose calls the host
+ * paces, add 72 or 80 bytes of their own (a call of one plain step: 3.4 us with 304
+ * bytes in all, 2.9 with 280). */
 struct StepConst {
     int d, n;
     int ni, nj, nk;     /* extents mapped onto (march axis, tile rows, tile columns) */
@@ -75,23 +80,25 @@ struct StepConst {
     /* the same coefficients rounded to float once on the host, so float kernels
      * read them straight from the parameter bank instead of converting per site */
     float c2f, c3f, c4f, v2f, v3f, v4f, dvf;
-    float dtf, dxf, dx2f, inv_dx2f;
-    double dx, dx2, inv_dx2;
-    int dx2_pow2;
-    double dxLD, mpl;
-    int alpha, expanding;
-    int want_local;
-    int force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
-    int temporal;       /* steps per pass for static 3-D lattices (1: no temporal blocking) */
-    /* fields below: behind those that the kernels load in groups of 16 bytes */
+    float dtf;
+    int odd;            /* the step's index is odd: expanding steps march the planes in turn forwards and
+                           backwards */
+    float dx2f, inv_dx2f;
     int pitch;          /* elements from a row of the last axis to the next: n, or (d = 3 runs) n rounded
                            up to whole 16-byte vectors. The pad holds the periodic images of the row's
                            first sites: every kernel that writes phi or pi keeps them equal */
-    int odd;            /* the step's index is odd: expanding steps march the planes in turn forwards and
-                           backwards */
-    int dx2_pair;       /* fma(x, inv_dx2_hi, x inv_dx2_lo) is x / dx2 rounded */
-    double inv_dx2_hi, inv_dx2_lo;   /* 1/dx2 as a pair (reciprocal_pair, cb_api.cpp) */
+    double dx, dx2;
+    double inv_dx2;     /* 1/dx2, rounded (dx2_pair: down) */
+    int dx2_pow2;
+    int dx2_pair;       /* fma(x, inv_dx2, x inv_dx2_lo) is x / dx2 rounded (reciprocal_pair, cb_api.cpp) */
+    double dxLD, mpl;
+    int alpha, expanding;
+    int want_local;
+    short force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
+    short temporal;       /* steps per pass for static 3-D lattices (1: no temporal blocking) */
+    double inv_dx2_lo;    /* 1/dx2 - inv_dx2, rounded */
 };
+static_assert((sizeof(StepConst) + 72) % 64 == 24, "dear to launch");
 
 bool reciprocal_pair(double d, double &zh, double &zl);
 

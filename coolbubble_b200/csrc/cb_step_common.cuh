@@ -111,7 +111,7 @@ enum { BY_MUL = 0, BY_PAIR = 1, BY_DIV = 2 };
 
 template <int BY>
 __device__ __forceinline__ double over_dx2(const StepConst &k, double lap) {
-    if (BY == BY_PAIR) return __fma_rn(lap, k.inv_dx2_hi, __dmul_rn(lap, k.inv_dx2_lo));
+    if (BY == BY_PAIR) return __fma_rn(lap, k.inv_dx2, __dmul_rn(lap, k.inv_dx2_lo));
     return BY == BY_MUL ? __dmul_rn(lap, k.inv_dx2) : __ddiv_rn(lap, k.dx2);
 }
 
