@@ -71,10 +71,26 @@ bool batched(const cb_handle *h) {
     return h->p.d == 2 && h->unit_scale && !h->k.force_generic && h->k.temporal != 1;
 }
 
-/* The member's buffers and record to the batch's array, starting from record
- * row `first` of the call. */
-cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev) {
+cudaError_t grow_partials(cb_ensemble::Batch &b, size_t rows) {
+    if (rows <= b.rows) return cudaSuccess;
+    if (b.partials) cudaFreeAsync(b.partials, b.stream);
+    b.partials = nullptr;
+    b.rows = 0;
+    const cudaError_t e = cudaMallocAsync((void **)&b.partials, rows * NSUM * sizeof(double), b.stream);
+    if (e == cudaSuccess) b.rows = rows;
+    return e;
+}
+
+/* The members' buffers, records of the call and, for launches of `steps` steps
+ * with sums (0: none), rows of partial sums to the batch's array. */
+cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev, int steps) {
     std::vector<Batch2Member> host(b.idx.size());
+    std::vector<int> tiles;
+    size_t rows = 0;
+    if (steps > 0) {
+        tiles = batch2_tiles(b.ns, b.prec, b.kind, steps);
+        if (tiles.empty()) return cudaErrorInvalidValue;
+    }
     for (size_t q = 0; q < b.idx.size(); ++q) {
         const cb_handle *h = e->members[b.idx[q]];
         Batch2Member &m = host[q];
@@ -86,24 +102,24 @@ cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev) {
         }
         m.st = h->st;
         m.records = e->records + (size_t)b.idx[q] * nev;
+        m.row = (int)rows;
+        if (steps > 0) rows += (size_t)tiles[q];
     }
+    const cudaError_t err = grow_partials(b, rows);
+    if (err != cudaSuccess) return err;
     return cudaMemcpyAsync(b.dev, host.data(), host.size() * sizeof(Batch2Member), cudaMemcpyHostToDevice, b.stream);
-}
-
-cudaError_t grow_partials(cb_ensemble::Batch &b, size_t rows) {
-    if (rows <= b.rows) return cudaSuccess;
-    if (b.partials) cudaFreeAsync(b.partials, b.stream);
-    b.partials = nullptr;
-    b.rows = 0;
-    const cudaError_t e = cudaMallocAsync((void **)&b.partials, rows * NSUM * sizeof(double), b.stream);
-    if (e == cudaSuccess) b.rows = rows;
-    return e;
 }
 
 /* All steps of a call for one batch: intervals of sums_every steps (the last
  * one may be shorter and has no line), each in launches of several steps. */
 cudaError_t run_batch(cb_ensemble *e, cb_ensemble::Batch &b, int nsteps, int sums_every, int nev) {
-    cudaError_t err = upload_members(e, b, nev);
+    /* every interval with a line is cut alike, so all launches with sums have the same steps */
+    int last = 0;
+    for (int left = nev > 0 ? sums_every : 0; left > 0; left -= last) {
+        last = batch2_steps(b.ns, b.prec, b.kind, left);
+        if (last < 1) return cudaErrorInvalidValue;
+    }
+    cudaError_t err = upload_members(e, b, nev, last);
     b.launches = 0;
     for (int done = 0, j = 0; done < nsteps && err == cudaSuccess;) {
         const int span = nev > 0 ? std::min(sums_every, nsteps - done) : nsteps - done;
@@ -111,11 +127,8 @@ cudaError_t run_batch(cb_ensemble *e, cb_ensemble::Batch &b, int nsteps, int sum
         for (int left = span; left > 0 && err == cudaSuccess;) {
             const int t = batch2_steps(b.ns, b.prec, b.kind, left);
             if (t < 1) return cudaErrorInvalidValue;
-            const bool sums = line && t == left;
-            if (sums) err = grow_partials(b, batch2_partial_rows(b.ns, b.prec, b.kind, t));
-            if (err == cudaSuccess)
-                err = launch_step2_batch(b.prec, b.kind, b.dev, b.ns, t, b.launches & 1, sums ? j : -1, b.partials,
-                                         b.stream);
+            err = launch_step2_batch(b.prec, b.kind, b.dev, b.ns, t, b.launches & 1, line && t == left ? j : -1,
+                                     b.partials, b.stream);
             b.launches++;
             left -= t;
         }

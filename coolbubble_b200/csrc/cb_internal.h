@@ -162,15 +162,18 @@ cudaError_t launch_step2_tb(int prec, const StepConst &k, int steps, bool sums, 
 /* Many static d = 2 lattices of one precision and kind per launch: steps at a
  * time (batch2_steps of the `left` to come), the last with sums into record
  * `event` of each (< 0: none). flip: which of a member's buffers hold the
- * fields now; partials: batch2_partial_rows rows. ns: the members' n. */
+ * fields now. ns: the members' n, largest first. partials: as many rows as all
+ * members have tiles (batch2_tiles, of a launch of so many steps), a member's
+ * from its `row` on. */
 struct Batch2Member {
     StepConst k;
     void *phi[2], *pi[2];
     DevState *st, *records;
+    int row;
 };
 int batch2_kind(const StepConst &k, int prec);   /* members of a launch share it: form of the rows, division by dx^2 */
 int batch2_steps(const std::vector<int> &ns, int prec, int kind, int left);
-size_t batch2_partial_rows(const std::vector<int> &ns, int prec, int kind, int steps);
+std::vector<int> batch2_tiles(const std::vector<int> &ns, int prec, int kind, int steps);
 cudaError_t launch_step2_batch(int prec, int kind, const Batch2Member *members, const std::vector<int> &ns, int steps,
                                int flip, int event, double *partials, cudaStream_t s);
 

@@ -39,6 +39,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 #include <vector>
 
@@ -404,11 +405,13 @@ __global__ void __launch_bounds__(TB2_MAXW * 32, 1)
     if (SUMS) finish_sums(k, acc, st, partials, blockIdx.x, gridDim.x, nullptr);
 }
 
+constexpr size_t BATCH2_MOST = 65535;   /* lattices of a launch: gridDim.y */
+
 /* One launch of `steps` steps over many lattices of one kind (ensembles):
  * block (x, y) takes tile x of lattice y, where it has one. */
 template <typename T, int K, int FORM, int BY, bool SUMS>
 __global__ void __launch_bounds__(TB2_MAXW * 32, 1)
-    k_step2_batch(const Batch2Member *__restrict__ members, Tiles g0, int steps, int flip, int event, int max_tiles,
+    k_step2_batch(const Batch2Member *__restrict__ members, Tiles g0, int steps, int flip, int event,
                   double *partials) {
     using VV = Vec<T>;
     using V = typename VV::V;
@@ -468,8 +471,7 @@ __global__ void __launch_bounds__(TB2_MAXW * 32, 1)
                                          static_cast<T *>(mb.phi[1 - flip]), static_cast<T *>(mb.pi[1 - flip]));
     pdl_allow_next();
     if (SUMS)
-        finish_sums(k, acc, mb.st, partials + (size_t)blockIdx.y * max_tiles * NSUM, blockIdx.x, g.tiles,
-                    mb.records + event);
+        finish_sums(k, acc, mb.st, partials + (size_t)mb.row * NSUM, blockIdx.x, g.tiles, mb.records + event);
 }
 
 }  // namespace
@@ -554,8 +556,8 @@ bool plan_2d(const StepConst &k, int prec, int steps, Plan2 &p) {
     }, p);
 }
 
-/* the tiles of lattices of these sizes, and of the one with most */
-bool plan_batch(const std::vector<int> &ns, int prec, int form, int steps, Plan2 &p, int *max_tiles) {
+/* the tiles of lattices of these sizes; each: of every one of them (may be NULL) */
+bool plan_batch(const std::vector<int> &ns, int prec, int form, int steps, Plan2 &p, std::vector<int> *each) {
     const int W = prec == P_FP64 ? 2 : 4;
     if (!plan_tiles(prec, form, steps, [&](Tiles &g, int h) -> long long {
             long long all = 0;
@@ -569,15 +571,15 @@ bool plan_batch(const std::vector<int> &ns, int prec, int form, int steps, Plan2
                 if (of_last == 0) return 0;
                 all += of_last;
             }
-            return all;
+            return all <= INT_MAX ? all : 0;
         }, p))
         return false;
-    if (max_tiles) {
-        *max_tiles = 0;
+    if (each) {
+        each->clear();
         for (int n : ns) {
             Tiles g = p.g;
             g.ty = p.rows * p.warps - 2 * steps;
-            *max_tiles = std::max(*max_tiles, (int)tiles_of_one(g, n, W, form, steps, p.rows * p.warps));
+            each->push_back((int)tiles_of_one(g, n, W, form, steps, p.rows * p.warps));
         }
     }
     return true;
@@ -700,10 +702,11 @@ int batch2_steps(const std::vector<int> &ns, int prec, int kind, int left) {
     });
 }
 
-size_t batch2_partial_rows(const std::vector<int> &ns, int prec, int kind, int steps) {
+std::vector<int> batch2_tiles(const std::vector<int> &ns, int prec, int kind, int steps) {
     Plan2 p;
-    int most = 0;
-    return plan_batch(ns, prec, kind % 3, steps, p, &most) ? (size_t)most * ns.size() : 0;
+    std::vector<int> each;
+    plan_batch(ns, prec, kind % 3, steps, p, &each);
+    return each;
 }
 
 int batch2_kind(const StepConst &k, int prec) {
@@ -714,14 +717,20 @@ int batch2_kind(const StepConst &k, int prec) {
 cudaError_t launch_step2_batch(int prec, int kind, const Batch2Member *members, const std::vector<int> &ns, int steps,
                                int flip, int event, double *partials, cudaStream_t s) {
     Plan2 p;
-    int most = 0;
-    if (steps < 1 || ns.empty() || !plan_batch(ns, prec, kind % 3, steps, p, &most)) return cudaErrorInvalidValue;
+    std::vector<int> tiles;
+    if (steps < 1 || ns.empty() || !plan_batch(ns, prec, kind % 3, steps, p, &tiles)) return cudaErrorInvalidValue;
     const size_t smem = (size_t)2 * 64 * p.warps * 16;
     auto go = [&](auto t, auto rows, auto al, auto dv, auto su) -> cudaError_t {
         using T = decltype(t);
         auto fn = k_step2_batch<T, decltype(rows)::value, decltype(al)::value, decltype(dv)::value, decltype(su)::value>;
-        return launch_pdl(fn, dim3((unsigned)most, (unsigned)ns.size()), dim3(p.warps * 32), smem, s, members, p.g,
-                          steps, flip, event, most, partials);
+        /* a grid has at most 65535 lattices; the first of each is its largest */
+        for (size_t at = 0; at < ns.size(); at += BATCH2_MOST) {
+            const unsigned count = (unsigned)std::min(ns.size() - at, BATCH2_MOST);
+            const cudaError_t e = launch_pdl(fn, dim3((unsigned)tiles[at], count), dim3(p.warps * 32), smem, s,
+                                             members + at, p.g, steps, flip, event, partials);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
     };
     using std::integral_constant;
     using Yes = std::true_type;
