@@ -642,9 +642,16 @@ int step2tb_steps(const StepConst &k, int prec, int left, bool sums) {
     /* The start and the block-wide sums of a launch here are not earned back by the one
      * step of a small lattice (in us, double: 64^2 9.0, one-step kernel 7.7; 256^2 10.5
      * and 9.5; 320^2 11.2 and 11.3; 512^2 13.9 and 18.0), by two of a very small one
-     * (32^2 8.8 and 8.6; 64^2 9.4 and 9.3), nor where the strips' kernel has one per row
-     * (1024^2 float 17.0 and 13.7; with two, in double, 21.0 and 22.1). */
-    if (sums && ((left == 1 && (k.n <= 288 || step2_one_strip(k, prec))) || (left == 2 && k.n <= 64))) return 0;
+     * (32^2 8.8 and 8.6; 64^2 9.4 and 9.3), nor by one or two where the strips' kernel has
+     * one per row (1024^2 float 17.0 and 13.7; calls of two 43.1 and 36.6). Large lattices
+     * read their halo for one step only: strips from 4096^2 on in float and where double
+     * divides by the compiler's division (calls of one step, float: 3072^2 82.0 here, 81.3
+     * in strips; 3584^2 94 and 106; 4096^2 118 and 111; 8192^2 340 and 315; double that
+     * divides: 3584^2 153 and 154; 4096^2 191 and 180; 8192^2 638 and 597; other double
+     * 8192^2 576 and 597). */
+    const bool strip = step2_one_strip(k, prec);
+    const bool large = k.n >= 4096 && step2_applies(k, prec, false) && (prec != P_FP64 || !(k.dx2_pow2 || k.dx2_pair));
+    if (sums && ((left == 1 && (k.n <= 288 || strip || large)) || (left == 2 && (k.n <= 64 || strip)))) return 0;
     return even_split(left, [&](int t) {
         Plan2 p;
         return plan_2d(k, prec, t, p) ? p.us : 0.0;
