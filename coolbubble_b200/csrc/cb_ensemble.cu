@@ -16,7 +16,7 @@
  * 3.2 us per step and lattice), with lines every 40 steps 3.2 (6.6); 128 of
  * 64^2 1.4 us per step (2.1), 64 of 256^2 4.6 (6.7).
  *
- * Other members (d = 1, 3, a static background that did not start at a = 1)
+ * Other members (d = 1, 3, large lattices, a static background that did not start at a = 1)
  * are stepped by their own handles on their own streams, concurrently.
  */
 #include <cuda_runtime.h>
@@ -46,6 +46,17 @@ struct cb_ensemble {
         size_t rows = 0;
         cudaStream_t stream = nullptr;
         int launches = 0;              /* of the running call */
+        /* the plan, which only the members' sizes decide: steps of the next launch by the
+         * steps left of an interval, and every member's tiles in launches of tiles_of steps */
+        std::map<int, int> cut;
+        std::vector<int> tiles;
+        int tiles_of = 0;
+        int next(int left) {
+            if (left > 1024) return batch2_steps(ns, prec, kind, left);   /* the plan kept stays small */
+            int &t = cut[left];
+            if (t == 0) t = batch2_steps(ns, prec, kind, left);
+            return t;
+        }
     };
     std::vector<Batch> batches;
     std::vector<int> own;              /* members stepped by their own handles */
@@ -67,8 +78,16 @@ int size_class(int prec, int d, int n) {
     return 0;
 }
 
+/* Members stepped in batches. A large lattice fills the GPU by itself, and its own
+ * launches choose kernel and depth for it alone: in double from 2048^2 on, in float
+ * from 3072^2 (one member, us in a batch and on its own stream; ten steps with a line
+ * each: double 1448^2 491 and 400, 2048^2 752 and 464, 8192^2 9472 and 4560, float
+ * 2048^2 524 and 370, 3072^2 738 and 670, 8192^2 5388 and 2974; 40 steps and one line:
+ * double 2048^2 547 and 499, float 2048^2 214 and 214; 40 plain steps: double 2048^2
+ * 488 and 466, float 2048^2 170 and 180, 3072^2 347 and 347). */
 bool batched(const cb_handle *h) {
-    return h->p.d == 2 && h->unit_scale && !h->k.force_generic && h->k.temporal != 1;
+    const int most = h->prec == P_FP64 ? 2048 : 3072;
+    return h->p.d == 2 && h->p.n_grids < most && h->unit_scale && !h->k.force_generic && h->k.temporal != 1;
 }
 
 cudaError_t grow_partials(cb_ensemble::Batch &b, size_t rows) {
@@ -85,12 +104,12 @@ cudaError_t grow_partials(cb_ensemble::Batch &b, size_t rows) {
  * with sums (0: none), rows of partial sums to the batch's array. */
 cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev, int steps) {
     std::vector<Batch2Member> host(b.idx.size());
-    std::vector<int> tiles;
     size_t rows = 0;
-    if (steps > 0) {
-        tiles = batch2_tiles(b.ns, b.prec, b.kind, steps);
-        if (tiles.empty()) return cudaErrorInvalidValue;
+    if (steps > 0 && steps != b.tiles_of) {
+        b.tiles = batch2_tiles(b.ns, b.prec, b.kind, steps);
+        b.tiles_of = steps;
     }
+    if (steps > 0 && b.tiles.empty()) return cudaErrorInvalidValue;
     for (size_t q = 0; q < b.idx.size(); ++q) {
         const cb_handle *h = e->members[b.idx[q]];
         Batch2Member &m = host[q];
@@ -103,7 +122,7 @@ cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev, int s
         m.st = h->st;
         m.records = e->records + (size_t)b.idx[q] * nev;
         m.row = (int)rows;
-        if (steps > 0) rows += (size_t)tiles[q];
+        if (steps > 0) rows += (size_t)b.tiles[q];
     }
     const cudaError_t err = grow_partials(b, rows);
     if (err != cudaSuccess) return err;
@@ -115,17 +134,15 @@ cudaError_t upload_members(cb_ensemble *e, cb_ensemble::Batch &b, int nev, int s
 cudaError_t run_batch(cb_ensemble *e, cb_ensemble::Batch &b, int nsteps, int sums_every, int nev) {
     /* every interval with a line is cut alike, so all launches with sums have the same steps */
     int last = 0;
-    for (int left = nev > 0 ? sums_every : 0; left > 0; left -= last) {
-        last = batch2_steps(b.ns, b.prec, b.kind, left);
-        if (last < 1) return cudaErrorInvalidValue;
-    }
+    for (int left = nev > 0 ? sums_every : 0; left > 0; left -= last)
+        if ((last = b.next(left)) < 1) return cudaErrorInvalidValue;
     cudaError_t err = upload_members(e, b, nev, last);
     b.launches = 0;
     for (int done = 0, j = 0; done < nsteps && err == cudaSuccess;) {
         const int span = nev > 0 ? std::min(sums_every, nsteps - done) : nsteps - done;
         const bool line = nev > 0 && span == sums_every && j < nev;
         for (int left = span; left > 0 && err == cudaSuccess;) {
-            const int t = batch2_steps(b.ns, b.prec, b.kind, left);
+            const int t = b.next(left);
             if (t < 1) return cudaErrorInvalidValue;
             err = launch_step2_batch(b.prec, b.kind, b.dev, b.ns, t, b.launches & 1, line && t == left ? j : -1,
                                      b.partials, b.stream);
@@ -230,16 +247,8 @@ int cb_ensemble_step(cb_ensemble *e, int nsteps, int sums_every, cb_sums *out) {
         std::vector<double> t_start(count);
         for (int i = 0; i < count; ++i) t_start[i] = e->members[i]->t;
         cudaError_t err = cudaSuccess;
-        for (auto &b : e->batches) {
-            /* whatever the members still have queued on their own streams comes first */
-            for (int i : b.idx)
-                if (err == cudaSuccess && cudaStreamQuery(e->members[i]->stream) != cudaSuccess) {
-                    cudaGetLastError();
-                    err = cudaStreamSynchronize(e->members[i]->stream);
-                }
-            if (err == cudaSuccess) err = run_batch(e, b, nsteps, sums_every, nev);
-        }
-        /* the others: their own step kernels on their own streams, records copied on the device */
+        /* first the members with streams of their own, which then step while the host gets
+         * to the batches; records copied on the device */
         for (int i : e->own) {
             if (err != cudaSuccess) break;
             cb_handle *h = e->members[i];
@@ -257,6 +266,16 @@ int cb_ensemble_step(cb_ensemble *e, int nsteps, int sums_every, cb_sums *out) {
                 }
                 done += kk;
             }
+        }
+        for (auto &b : e->batches) {
+            if (err != cudaSuccess) break;
+            /* whatever the members still have queued on their own streams comes first */
+            for (int i : b.idx)
+                if (err == cudaSuccess && cudaStreamQuery(e->members[i]->stream) != cudaSuccess) {
+                    cudaGetLastError();
+                    err = cudaStreamSynchronize(e->members[i]->stream);
+                }
+            if (err == cudaSuccess) err = run_batch(e, b, nsteps, sums_every, nev);
         }
         /* every stream drains even after an error: the members' buffers must not be in use */
         for (auto &b : e->batches) {

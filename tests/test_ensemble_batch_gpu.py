@@ -43,3 +43,29 @@ def test_batched_members_equal_their_solo_runs(prec):
         np.testing.assert_array_equal(fa["phi"], fb["phi"], err_msg=str(specs[i]))
         np.testing.assert_array_equal(fa["pi"], fb["pi"], err_msg=str(specs[i]))
         assert m.sums()["t"] == s.sums()["t"] and m.counters()[1] == s.counters()[1]
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32c"])
+def test_large_members_step_as_their_solo_runs(prec):
+    """A lattice that fills the GPU by itself takes its own launches, beside the
+    batch of the small ones."""
+    import coolbubble_b200 as cb
+    from coolbubble_b200.ensemble import Ensemble
+    made = []
+    for n in (2048 if prec == "fp64" else 3072, 64, 64):
+        p = cb.make_params(2, n, n / 8.0, 4.0, 0.0125, precision=prec, memorysave=1)
+        rng = np.random.default_rng(n)
+        made.append((p, 0.3 + 0.1 * rng.random(n * n), 0.05 * rng.standard_normal(n * n)))
+    mix, solo = [cb.Bubble(*m) for m in made], [cb.Bubble(*m) for m in made]
+    ens = Ensemble(mix)
+    for nsteps, every in ((6, 1), (40, 40)):
+        lines = ens.step(nsteps, every)
+        for got, s in zip(lines, solo):
+            want = [s.step(every, sums=True) for _ in range(nsteps // every)]
+            for a, b in zip(got, want):
+                assert a["t"] == b["t"] and abs(a["etot"] - b["etot"]) <= s.N * 2.0 ** -52 * abs(b["etot"])
+    assert mix[0].counters() == solo[0].counters()
+    for m, s in zip(mix, solo):
+        fa, fb = m.fields(), s.fields()
+        for key in ("phi", "pi"):
+            np.testing.assert_array_equal(fa[key], fb[key])
