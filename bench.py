@@ -517,12 +517,12 @@ def ensemble_measure(steps, warmup, seed, dist=None):
         el = max_over_ranks(dist, time.perf_counter() - t0)
         out[prec] = dict(seconds=el, value=ws * sites * steps / el, plans=plans)
         del ens, runs
-    resident = sum(1 for c, _ in out["fp32c"]["plans"] if c > 0)
+    batched = sum(1 for _, threads in out["fp32c"]["plans"] if threads > 0)
     return {
         "value": out["fp32c"]["value"], "unit": "site-updates/s", "steps": steps,
         "ms_per_step": 1e3 * out["fp32c"]["seconds"] / steps, "members": len(specs), "sites_per_step": sites,
         "n_mix": {str(m): sum(1 for s in specs if s["n"] == m) for m in (128, 256, 512)},
-        "thermal_members": sum(1 for s in specs if s["thermal"]), "resident_members_fp32c": resident,
+        "thermal_members": sum(1 for s in specs if s["thermal"]), "batched_members_fp32c": batched,
         "fp64_value": out["fp64"]["value"], "speedup_vs_fp64": out["fp32c"]["value"] / out["fp64"]["value"],
         "hbm_equivalent_gbs": out["fp32c"]["value"] * 16 / 1e9,
         "timing": "host wall clock around one cb_ensemble_step call (launch, all steps, lines back)",

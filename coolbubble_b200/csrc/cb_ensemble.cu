@@ -67,7 +67,8 @@ struct cb_ensemble {
 namespace {
 
 /* The size class of a 2-D lattice: how many 200 KB shares (1, 2, 4, 8, 16)
- * three of its fields fill in whole rows; 0 beyond, or for other rows. */
+ * three of its fields fill in whole rows; 0 beyond, or for other rows. A way for
+ * callers to tell sizes apart; no launch depends on it. */
 int size_class(int prec, int d, int n) {
     const size_t esz = prec == P_FP64 ? 8 : 4;
     if (d != 2 || n % (16 / esz) != 0) return 0;
@@ -77,6 +78,8 @@ int size_class(int prec, int d, int n) {
     }
     return 0;
 }
+
+constexpr int LONG_INTERVAL = 64;   /* steps whose launches cb_ensemble_member_plan speaks of */
 
 /* Members stepped in batches. A large lattice fills the GPU by itself, and its own
  * launches choose kernel and depth for it alone: in double from 2048^2 on, in float
@@ -202,12 +205,18 @@ int cb_ensemble_create(int count, cb_handle *const *members, cb_ensemble **out) 
 }
 
 int cb_ensemble_member_plan(cb_ensemble *e, int m, int *cluster, int *threads) {
-    if (!e || m < 0 || m >= (int)e->members.size() || !cluster || !threads)
-        return fail(nullptr, CB_EINVAL, "cb_ensemble_member_plan: bad arguments");
-    const cb_handle *h = e->members[m];
-    *cluster = batched(h) ? size_class(h->prec, h->p.d, h->p.n_grids) : 0;
-    *threads = *cluster > 0 ? 256 : 0;
-    return CB_OK;
+    return cb::guard(nullptr, [&]() -> int {
+        if (!e || m < 0 || m >= (int)e->members.size() || !cluster || !threads)
+            return fail(nullptr, CB_EINVAL, "cb_ensemble_member_plan: bad arguments");
+        *cluster = *threads = 0;
+        for (auto &b : e->batches)
+            if (std::find(b.idx.begin(), b.idx.end(), m) != b.idx.end()) {
+                const cb_handle *h = e->members[m];
+                *cluster = size_class(h->prec, h->p.d, h->p.n_grids);
+                *threads = batch2_threads(b.ns, b.prec, b.kind, b.next(LONG_INTERVAL));
+            }
+        return CB_OK;
+    });
 }
 
 int cb_ensemble_destroy(cb_ensemble *e) {

@@ -173,6 +173,7 @@ struct Batch2Member {
 };
 int batch2_kind(const StepConst &k, int prec);   /* members of a launch share it: form of the rows, division by dx^2 */
 int batch2_steps(const std::vector<int> &ns, int prec, int kind, int left);
+int batch2_threads(const std::vector<int> &ns, int prec, int kind, int steps);   /* of a block */
 std::vector<int> batch2_tiles(const std::vector<int> &ns, int prec, int kind, int steps);
 cudaError_t launch_step2_batch(int prec, int kind, const Batch2Member *members, const std::vector<int> &ns, int steps,
                                int flip, int event, double *partials, cudaStream_t s);

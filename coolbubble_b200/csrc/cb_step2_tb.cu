@@ -716,6 +716,11 @@ std::vector<int> batch2_tiles(const std::vector<int> &ns, int prec, int kind, in
     return each;
 }
 
+int batch2_threads(const std::vector<int> &ns, int prec, int kind, int steps) {
+    Plan2 p;
+    return plan_batch(ns, prec, kind % 3, steps, p, nullptr) ? p.warps * 32 : 0;
+}
+
 int batch2_kind(const StepConst &k, int prec) {
     const int by = prec != P_FP64 || k.dx2_pow2 ? BY_MUL : k.dx2_pair ? BY_PAIR : BY_DIV;
     return by * 3 + form_of(k, prec);

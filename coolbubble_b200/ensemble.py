@@ -34,6 +34,7 @@ class Ensemble:
         self._h = None
 
     def plan(self, m):
+        """(size class of a batched member's lattice, threads of a block of its batch); 0 threads: on its own stream."""
         cs, nt = C.c_int(), C.c_int()
         check(L.lib.cb_ensemble_member_plan(self._h, m, C.byref(cs), C.byref(nt)))
         return cs.value, nt.value

@@ -291,10 +291,11 @@ int cb_ensemble_create(int count, cb_handle *const *members, cb_ensemble **out);
  * sums_every-th step of member m goes to out[m * (nsteps / sums_every) + j]. */
 int cb_ensemble_step(cb_ensemble *e, int nsteps, int sums_every, cb_sums *out);
 
-/* The size class of a batched member -- the shares of 200 KB (1, 2, 4, 8, 16)
- * that three of its fields fill in whole rows -- and the threads of a block;
- * 0, 0 for members larger than a class, with other rows, or stepped on their
- * own. */
+/* How member m is stepped. *threads: the threads of a block in its batch's
+ * launches (of intervals of 64 steps), 0 for a member stepped on its own stream.
+ * *cluster: the size class of a batched member's lattice -- the shares of 200 KB (1,
+ * 2, 4, 8, 16) that three of its fields fill in whole rows, 0 beyond or for other
+ * rows; it tells sizes apart, no launch depends on it. */
 int cb_ensemble_member_plan(cb_ensemble *e, int m, int *cluster, int *threads);
 
 int cb_ensemble_destroy(cb_ensemble *e);

@@ -69,3 +69,22 @@ def test_large_members_step_as_their_solo_runs(prec):
         fa, fb = m.fields(), s.fields()
         for key in ("phi", "pi"):
             np.testing.assert_array_equal(fa[key], fb[key])
+
+
+def test_plan_tells_which_members_are_batched():
+    """Threads of a block for every member of a batch, one number per batch, whatever
+    its size class; none for members on their own streams."""
+    import coolbubble_b200 as cb
+    from coolbubble_b200.ensemble import Ensemble
+
+    def run(d, n, prec):
+        p = cb.make_params(d, n, n / 8.0, 4.0, 0.0125, precision=prec, memorysave=1)
+        return cb.Bubble(p, np.zeros(n ** d))
+
+    runs = [run(2, 1000, "fp32c"), run(2, 64, "fp32c"), run(2, 400, "fp32c"), run(2, 250, "fp64"), run(2, 2048, "fp64"),
+            run(3, 16, "fp64"), run(1, 64, "fp64")]
+    plans = [Ensemble(runs).plan(i) for i in range(len(runs))]
+    assert all(threads in (128, 256, 512) for _, threads in plans[:4])
+    assert plans[0][0] == 0                     # beyond the classes, and batched all the same
+    assert plans[0][1] == plans[2][1]           # one batch: rows of vectors, float
+    assert plans[4:] == [(0, 0)] * 3
