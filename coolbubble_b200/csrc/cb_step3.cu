@@ -188,9 +188,11 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     constexpr bool UNI = DF || SUMS != SUM_NONE;       /* consumers leave together */
     constexpr bool FULL = SUMS == SUM_FULL || SUMS == SUM_LINE;
     constexpr int NS = FULL ? NSUM : 3;                /* sums carried (S_EK, S_EP, S_EG first) */
-    /* float with padded rows: the full sums in double per vector (250^3: 69 us; the
-     * generic kernel, which compensates its sums per site, 180) */
-    constexpr bool DSUM = RAG && SUMS == SUM_FULL && std::is_same<T, float>::value;
+    /* float with padded rows: every site's term in double, as the generic kernel, which took
+     * them before, compensates each (a reporting step of 250^3 89 us; 69 with a vector's
+     * terms added in float first, 180 in the generic kernel; plain expanding steps of 250^3
+     * 52.6 and 52.3 with the Friedmann sums' pairs added in float) */
+    constexpr bool DSUM = RAG && SUMS != SUM_NONE && std::is_same<T, float>::value;
     extern __shared__ __align__(128) unsigned char smraw[];
     const int n = NV ? NV * W : k.n, np = RAG ? k.pitch : n;   /* sites and elements of a row */
     const int tj = NV ? NV_TILE / NV : tj_;
@@ -533,7 +535,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                          * instruction per pair), the same operations in the same order as
                          * the scalar path for the fields; the sums of a pair's two sites
                          * are added pairwise over the vector, then its sum enters the
-                         * compensated per-thread accumulator */
+                         * compensated per-thread accumulator (padded rows: DSUM) */
                         const F2 c01 = f2_pack(c.x, c.y), c23 = f2_pack(c.z, c.w);
                         const F2 km01 = f2_pack(left, c.x), mid = f2_pack(c.y, c.z), kp23 = f2_pack(c.w, right);
                         F2 phi01, pi01, phi23, pi23;
@@ -609,8 +611,10 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                                         x = f2_mul(x, x);
                                         y = f2_mul(y, y);
                                     }
-                                    x = f2_add(x, y);
-                                    dacc[q] = __dadd_rn(dacc[q], (double)(f2_lo(x) + f2_hi(x)));
+                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_lo(x));
+                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_hi(x));
+                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_lo(y));
+                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_hi(y));
                                 } else
                                 /* the energies (and the previous half step's kinetic sum, which
                                  * enters the time-centred Ekin) are compensated, per half of the
