@@ -952,7 +952,10 @@ int cb_get_fields_f32(cb_handle *h, float *phi, float *pi, float *ekin, float *e
             from = h->tmp;
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(dst[f], from, h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
-        if (e != cudaSuccess) return cuda_fail(h, e, "downloading a field");
+        if (e != cudaSuccess) {
+            cudaStreamSynchronize(h->stream);   /* the fields before it are still on their way to the caller */
+            return cuda_fail(h, e, "downloading a field");
+        }
     }
     if ((r = sync(h, "downloading the fields")) != CB_OK) return r;
     return CB_OK;

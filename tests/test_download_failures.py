@@ -1,0 +1,28 @@
+"""Downloads that fail half-way, on a fake of the CUDA runtime (no GPU): what the
+caller's buffers may hold and whether anything still writes to them."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "coolbubble_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("fake") / "fake_cuda")
+    cuda = os.environ.get("CUDA", "/usr/local/cuda")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I" + CSRC, "-I" + os.path.join(ROOT, "include"),
+                    "-I" + os.path.join(cuda, "include"), os.path.join(ROOT, "tests", "native", "fake_cuda.cpp"),
+                    os.path.join(CSRC, "cb_api.cpp"), os.path.join(CSRC, "cb_pool.cpp"), "-o", exe, "-lpthread"], check=True)
+    return exe
+
+
+def run(exe, what):
+    r = subprocess.run([exe, what], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout == "ok\n", r.stdout + r.stderr
+
+
+def test_a_failed_download_leaves_no_copy_under_way(fake):
+    run(fake, "download")
