@@ -70,7 +70,7 @@ void spread(size_t bytes, F part) {
 }
 
 /* A field kept for the caller. Its memory is not cleared before the download
- * fills it, lies on large pages where the system grants them and is touched by
+ * fills it (so only a completed run's is handed out), lies on large pages where the system grants them and is touched by
  * several threads: two fields of 192^3 cost the stepping thread 22 ms as
  * zero-filled vectors and 8 this way, and collecting them 13 and 6 ms. */
 struct HostField {
@@ -525,8 +525,15 @@ int cb_pool_result(cb_pool *P, int64_t id, cb_sums *lines, int max_lines, int *n
     if (nlines) *nlines = (int)r->lines.size();
     if (lines)
         for (int i = 0; i < (int)r->lines.size() && i < max_lines; ++i) lines[i] = r->lines[i];
-    if (phi && r->phi.p) r->phi.copy_to(phi);
-    if (pi && r->pi.p) r->pi.copy_to(pi);
+    /* a failed run's fields may be half downloaded, over what their memory held before */
+    const bool done = r->state == CB_REQ_DONE;
+    auto give = [done](const HostField &f, float *to) {
+        if (!to || !f.p) return;
+        if (done) f.copy_to(to);
+        else std::memset(to, 0, f.n * sizeof(float));
+    };
+    give(r->phi, phi);
+    give(r->pi, pi);
     if (latency_s) *latency_s = seconds(r->t_submit, r->t_done);
     if (err && err_cap) {
         std::strncpy(err, r->err.c_str(), err_cap - 1);

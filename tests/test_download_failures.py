@@ -26,3 +26,7 @@ def run(exe, what):
 
 def test_a_failed_download_leaves_no_copy_under_way(fake):
     run(fake, "download")
+
+
+def test_a_served_run_without_its_fields_hands_out_zeros(fake):
+    run(fake, "served")
