@@ -222,6 +222,14 @@ inline size_t field_elems(const StepConst &k) {
     for (int i = 1; i < k.d; ++i) e *= (size_t)k.n;
     return e;
 }
+/* Rows of n elements in tiles of t rows on the marching kernels, two vectors a thread (u and
+ * u + half the tile's): whether every warp's vectors are consecutive in one row, all tiles are
+ * whole, and both vectors of a thread start at the same site of their rows -- half a tile is
+ * then whole rows, so t is even. One set of row-end offsets serves both. */
+inline bool whole_rows(int n, int pitch, int prec, int t) {
+    const int W = prec == 0 ? 2 : 4;
+    return pitch == n && n % W == 0 && n / W % 32 == 0 && t % 2 == 0 && n % t == 0;
+}
 /* a d = 3 run's row pitch: whole 16-byte vectors where the staged kernels apply */
 inline int run_pitch(int d, int n, int prec) {
     const int W = prec == 0 ? 2 : 4;

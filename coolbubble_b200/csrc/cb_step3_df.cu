@@ -543,7 +543,7 @@ bool plan_df(const StepConst &k, int prec, PlanDF &best) {
         const int threads = (t * nv + 63) / 64 * 32;
         const size_t stage = 2 * (size_t)(t + 2) * row;
         if (threads > DF_MAXT || 4 * stage > budget) break;
-        const bool whole = k.pitch == n && nv % 32 == 0 && n % t == 0 && t * nv == 2 * threads;
+        const bool whole = whole_rows(n, k.pitch, prec, t);
         const double round = (0.55 + 0.05 * ((threads + 127) / 128 * 4)) * (whole ? 1.0 : 1.08);
         const long long ntiles = (n + t - 1) / t;
         for (long long w = 1; w <= 6; ++w) {

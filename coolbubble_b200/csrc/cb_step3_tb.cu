@@ -549,7 +549,7 @@ bool step3tb_geometry(const StepConst &k, int prec, int tl, int &tj, int &nstage
         const long long ntiles = (n + t - 1) / t;
         const int per_sched = (t * nv + 255) / 256;   /* warps per scheduler, two vectors each */
         /* rows of whole warps in whole tiles save the masks and per-slot wraps (launch below) */
-        const bool whole = np == n && nv % 32 == 0 && n % t == 0 && t * nv % 64 == 0;
+        const bool whole = whole_rows(n, np, prec, t);
         const double round = (whole ? 1.0 : 1.15) + (prec == P_FP64 ? 0.05 : 0.036) * (4.0 * per_sched + (2 * nv + 127) / 128);
         for (long long w = 1; w <= 8; ++w) {
             const long long P = std::min<long long>(w * slots / ntiles, n / 4);
@@ -587,7 +587,7 @@ cudaError_t launch_step3_tb(int prec, const StepConst &k, int tl, const void *ph
      * Other rows spread them as one pair of floats or one double per thread where the
      * threads suffice (250^3 float 29.3 us per step with whole vectors on some of the
      * warps, 28.4 with pairs, 31.5 site by site; 200^3 double 34.9 -> 33.7) */
-    const bool whole = k.pitch == k.n && (k.n / W) % 32 == 0 && k.n % tj == 0 && npos == 2 * nc;
+    const bool whole = whole_rows(k.n, k.pitch, prec, tj);
     auto go = [&](auto t, auto by, auto hw, auto wh) -> cudaError_t {
         using T = decltype(t);
         constexpr int HW = decltype(hw)::value;
