@@ -736,7 +736,7 @@ def main():
         "config": workload_config(args.workload, w),
         "details": {"precision": prec, "parallelism": f"replicas{ws}", "l2": l2_note(n, d, prec),
                     "steps_per_launch": args.steps / m["launches"],
-                    "temporal_block": os.environ.get("CB_TEMPORAL_BLOCK", "autotuned"),
+                    "temporal_block": os.environ.get("CB_TEMPORAL_BLOCK", "2 where it applies"),
                     "warmup_requested": args.warmup,
                     "energy_lines_in_window": sum(1 for _, e in event_chunks(m["warmup"], args.steps) if e)},
         "hbm_gbs": m["achieved_gbs"],

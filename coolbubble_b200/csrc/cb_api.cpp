@@ -13,7 +13,6 @@
 #include <cstdlib>
 #include <cstdint>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <new>
 #include <string>
@@ -186,10 +185,13 @@ StepConst make_const(const cb_params *p) {
     k.want_local = 0;
     const char *path = std::getenv("CB_STEP_PATH");
     k.force_generic = (path && std::string(path) == "generic") ? 1 : 0;
-    /* steps per pass of the static 3-D step: CB_TEMPORAL_BLOCK=1 or 2 fixes it;
-     * unset, it is chosen per lattice size by timing both passes once (0: not chosen yet) */
+    /* steps per launch of a static background: several, or with CB_TEMPORAL_BLOCK=1 one.
+     * Two-step passes are the faster ones wherever step3tb_geometry has them (us per step,
+     * one and two per pass, float: 125^3 8.9 and 7.3, 200^3 22.5 and 15.3, 257^3 54 and 32,
+     * 513^3 339 and 247, 768^3 1105 and 684; double: 64^3 7.1 and 5.5, 66^3 7.5 and 7.3,
+     * 144^3 17.9 and 15.6, 300^3 142 and 125, 400^3 320 and 314) */
     const char *tb = std::getenv("CB_TEMPORAL_BLOCK");
-    k.temporal = (short)(tb ? std::min(std::max(1, std::atoi(tb)), 99) : 0);
+    k.temporal = (short)(tb ? std::min(std::max(1, std::atoi(tb)), 99) : 2);
     if (k.force_generic) k.temporal = 1;
     return k;
 }
@@ -444,60 +446,6 @@ int ensure_tmp(cb_handle *h, size_t bytes) {
     return CB_OK;
 }
 
-/* The temporal-block autotuner: for a static 3-D run whose lattice the
- * two-step pass can take, time one-step and two-step passes on the run's own
- * stream (each reads the current fields and writes the spare buffers, so the
- * run's state does not change) and keep whichever moves a step faster; the
- * choice is cached per device, lattice size and precision. Both passes give the same
- * fields bit for bit, so the choice only changes the speed. */
-int choose_temporal(cb_handle *h) {
-    if (h->expanding || !h->unit_scale || h->p.d != 3) return 1;
-    int tj, ns, parts;
-    size_t sm;
-    unsigned g;
-    if (!step3tb_geometry(h->k, h->prec, 2, tj, ns, sm, g, parts)) return 1;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 1; }
-    static std::mutex mu;
-    static std::map<std::pair<int, int>, int> cache;
-    const std::pair<int, int> key(dev, 2 * h->p.n_grids + (h->prec == P_FP64 ? 1 : 0));
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = cache.find(key);
-        if (it != cache.end()) return it->second;
-    }
-    cudaEvent_t ev[3];
-    for (auto &x : ev)
-        if (cudaEventCreate(&x) != cudaSuccess) { cudaGetLastError(); return 1; }
-    const int i = h->cphi, j = h->cpi;
-    StepConst k = h->k;
-    k.want_local = 0;
-    auto one = [&]() {
-        return launch_step(h->prec, k, false, 0, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j], h->loc[0],
-                           h->loc[1], h->loc[2], h->st, h->partials, h->stream);
-    };
-    auto two = [&]() { return launch_step3_tb(h->prec, k, 2, h->phi[i], h->pi[j], h->phi[1 - i], h->pi[1 - j], h->st, h->stream); };
-    const int reps = 4;
-    cudaError_t e = one();
-    if (e == cudaSuccess) e = two();
-    if (e == cudaSuccess) e = cudaEventRecord(ev[0], h->stream);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = one();
-    if (e == cudaSuccess) e = cudaEventRecord(ev[1], h->stream);
-    for (int r = 0; r < reps && e == cudaSuccess; ++r) e = two();
-    if (e == cudaSuccess) e = cudaEventRecord(ev[2], h->stream);
-    if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
-    float t1 = 0.f, t2 = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&t1, ev[0], ev[1]);
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&t2, ev[1], ev[2]);
-    for (auto &x : ev) cudaEventDestroy(x);
-    if (e != cudaSuccess) { cudaGetLastError(); return 1; }
-    /* per step: t1 / reps against t2 / (2 reps); keep the two-step pass only for a clear gain */
-    const int tl = (t2 / 2.f < 0.97f * t1) ? 2 : 1;
-    std::lock_guard<std::mutex> lock(mu);
-    cache[key] = tl;
-    return tl;
-}
-
 /* Small lattices: a step's kernel takes less time than its launch, so chains
  * of GRAPH_STEPS plain steps (no sums reported; an expanding background's
  * Friedmann update stays on the device) are captured once into a CUDA graph
@@ -571,7 +519,6 @@ int step_impl(cb_handle *h, int nsteps, int flags, bool timed) {
     int tj, ns, parts;
     size_t sm;
     unsigned g;
-    if (h->p.d == 3 && h->k.temporal == 0 && nsteps > 2) h->k.temporal = (short)choose_temporal(h);
     const int tl = h->k.temporal;
     const bool tb_ok = !h->expanding && h->unit_scale && tl > 1 &&
                        step3tb_geometry(h->k, h->prec, tl, tj, ns, sm, g, parts);

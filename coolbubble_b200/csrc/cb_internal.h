@@ -95,7 +95,7 @@ struct StepConst {
     int alpha, expanding;
     int want_local;
     short force_generic;  /* 1: always use the generic tile kernel (diagnostics and cross-checks) */
-    short temporal;       /* steps per pass for static 3-D lattices (1: no temporal blocking) */
+    short temporal;       /* steps per pass of static 3-D lattices (1: one step per launch on every static lattice) */
     double inv_dx2_lo;    /* 1/dx2 - inv_dx2, rounded */
 };
 static_assert((sizeof(StepConst) + 72) % 64 == 24, "dear to launch");

@@ -1,7 +1,7 @@
 /* A CUDA runtime on the host for cb_api.cpp and cb_pool.cpp: "device" memory is
  * host memory, kernels do nothing, and copies to the host stay queued on their
  * stream until it is waited for. A test can make one of those copies fail. Built
- * and run by test_download_failures.py, which needs no GPU. */
+ * and run by test_host_path.py, which needs no GPU. */
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -25,6 +25,9 @@ std::mutex mu;
 std::vector<Copy> queued;
 size_t fail_bytes = 0;    /* copies to the host of this size count ... */
 int fail_at = -1;         /* ... and this one of them fails */
+
+int waits = 0, ones = 0, twos = 0;   /* waits for a stream or event, one-step and two-step launches */
+bool two_step = false;               /* the two-step pass applies */
 
 void run_stream(cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
@@ -67,14 +70,14 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, cudaMemcpyKind
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return *s = (cudaStream_t)std::malloc(1), cudaSuccess; }
 cudaError_t cudaStreamDestroy(cudaStream_t s) { return run_stream(s), std::free(s), cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t s) { return run_stream(s), cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t s) { return ++waits, run_stream(s), cudaSuccess; }
 /* an event is the stream it was recorded on */
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return *e = (cudaEvent_t)std::calloc(1, sizeof(cudaStream_t)), cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { return std::free(e), cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { return *(cudaStream_t *)e = s, cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t e) { return run_stream(*(cudaStream_t *)e), cudaSuccess; }
-cudaError_t cudaEventSynchronize(cudaEvent_t e) { return cudaEventQuery(e); }
+cudaError_t cudaEventSynchronize(cudaEvent_t e) { return ++waits, cudaEventQuery(e); }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.f, cudaSuccess; }
 cudaError_t cudaGetDevice(int *d) { return *d = 0, cudaSuccess; }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
@@ -106,7 +109,7 @@ size_t ic_blocks(const StepConst &) { return 1; }
 size_t step_blocks(const StepConst &) { return 1; }
 int step2tb_steps(const StepConst &, int, int, bool) { return 0; }
 bool step3df_applies(const StepConst &, int) { return false; }
-bool step3tb_geometry(const StepConst &, int, int, int &, int &, size_t &, unsigned &, int &) { return false; }
+bool step3tb_geometry(const StepConst &, int, int tl, int &, int &, size_t &, unsigned &, int &) { return two_step && tl == 2; }
 cudaError_t launch_convert(int, int, const void *, void *, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_flush_drift(int, const StepConst &, const void *, const void *, void *, DevState *, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_ic_backkick(int, const StepConst &, const void *, void *, DevState *, double *, cudaStream_t) { return cudaSuccess; }
@@ -114,7 +117,7 @@ cudaError_t launch_ic_energies(int, const StepConst &, const void *, const void 
                                cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_repitch(int, int, const void *, size_t, void *, size_t, int, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_step(int, const StepConst &, bool, int, const void *, const void *, void *, void *, void *, void *, void *,
-                        DevState *, double *, cudaStream_t) { return cudaSuccess; }
+                        DevState *, double *, cudaStream_t) { return ++ones, cudaSuccess; }
 cudaError_t launch_step2_tb(int, const StepConst &, int, bool, const void *, const void *, void *, void *, DevState *, double *,
                             cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_step3_df(int, const StepConst &, int, bool, void *, void *, void *, void *, DevState *, double *,
@@ -123,7 +126,7 @@ cudaError_t launch_step3_ms(int, const StepConst &, int, void *, void *, void *,
     return cudaErrorNotSupported;
 }
 cudaError_t launch_step3_tb(int, const StepConst &, int, const void *, const void *, void *, void *, DevState *, cudaStream_t) {
-    return cudaErrorNotSupported;
+    return ++twos, cudaSuccess;
 }
 }  // namespace cb
 
@@ -193,6 +196,24 @@ int served(int n, int which) {
     return cb_pool_destroy(pool) == CB_OK ? 0 : 1;
 }
 
+/* The first steps of a static 3-D run: the launches of those steps and no others,
+ * and no wait. */
+int first_steps(int n, int precision) {
+    const cb_params p = params(3, n, precision);
+    std::vector<double> start((size_t)n * n * n, 0.5);
+    cb_handle *h = nullptr;
+    two_step = true;
+    CHECK(cb_create_from_ic(&p, start.data(), nullptr, nullptr, &h) == CB_OK);
+    waits = ones = twos = 0;
+    CHECK(cb_step(h, 8, 0, nullptr) == CB_OK);
+    CHECK(waits == 0 && ones == 0 && twos == 4);
+    CHECK(cb_step(h, 3, 0, nullptr) == CB_OK);
+    CHECK(waits == 0 && ones == 1 && twos == 5);
+    int64_t launches = 0, steps = 0;
+    CHECK(cb_get_counters(h, &launches, &steps) == CB_OK && launches == 6 && steps == 11);
+    return cb_destroy(h) == CB_OK ? 0 : 1;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -200,6 +221,7 @@ int main(int argc, char **argv) {
     int bad = 0;
     if (what == "download") bad = download(2, 64, CB_FP32C) || download(2, 64, CB_FP64) || download(3, 65, CB_FP32C);
     else if (what == "served") bad = served(1500, 0) || served(1500, 1) || served(64, 1);
+    else if (what == "first") bad = first_steps(64, CB_FP64) || first_steps(65, CB_FP32C) || first_steps(128, CB_FP32C);
     else bad = std::printf("what?\n");
     std::printf(bad ? "failed\n" : "ok\n");
     return bad ? 1 : 0;

@@ -1,5 +1,5 @@
-"""Downloads that fail half-way, on a fake of the CUDA runtime (no GPU): what the
-caller's buffers may hold and whether anything still writes to them."""
+"""The library's host code on a fake of the CUDA runtime (no GPU): downloads that
+fail half-way, and what a run's first steps launch."""
 import os
 import subprocess
 
@@ -30,3 +30,7 @@ def test_a_failed_download_leaves_no_copy_under_way(fake):
 
 def test_a_served_run_without_its_fields_hands_out_zeros(fake):
     run(fake, "served")
+
+
+def test_first_steps_launch_their_steps_and_wait_for_nothing(fake):
+    run(fake, "first")
