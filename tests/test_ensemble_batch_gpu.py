@@ -88,3 +88,20 @@ def test_plan_tells_which_members_are_batched():
     assert plans[0][0] == 0                     # beyond the classes, and batched all the same
     assert plans[0][1] == plans[2][1]           # one batch: rows of vectors, float
     assert plans[4:] == [(0, 0)] * 3
+
+
+def test_batched_members_that_divide_by_division_equal_their_solo_runs():
+    """dx^2 without a two-operation division: a batch of its own."""
+    import coolbubble_b200 as cb
+    from coolbubble_b200.ensemble import Ensemble
+    made = []
+    for i, n in enumerate((64, 200, 101, 500)):
+        p = cb.make_params(2, n, n * 0.17, 4.0, 0.017, precision="fp64", memorysave=1)
+        made.append((p, 0.3 + smooth_noise(2, n, 0.1, seed=i), smooth_noise(2, n, 0.05, seed=50 + i)))
+    mix, solo = [cb.Bubble(*m) for m in made], [cb.Bubble(*m) for m in made]
+    Ensemble(mix).step(23, 0)
+    for m, s in zip(mix, solo):
+        s.step(23, sums=False)
+        a, b = m.fields(), s.fields()
+        for key in ("phi", "pi"):
+            np.testing.assert_array_equal(a[key], b[key])

@@ -30,3 +30,25 @@ def test_two_step_pass_equals_one_step_passes(n, L, prec, monkeypatch):
         np.testing.assert_array_equal(fa["phi"], fb["phi"])
         np.testing.assert_array_equal(fa["pi"], fb["pi"])
     assert two.counters() == (1 + 4 + 3, 13) and one.counters() == (13, 13)
+
+
+@pytest.mark.parametrize("dx", [0.1, 0.125])
+def test_two_step_pass_of_128_vectors_a_row_in_double(dx, monkeypatch):
+    """256^3 in double, rows whose shared offsets are constants of the kernel:
+    dx^2 that divides in two operations and in one."""
+    import coolbubble_b200 as cb
+    n = 256
+    rng = np.random.default_rng(5)
+    start = 0.4 + 0.1 * rng.standard_normal(n ** 3), 0.05 * rng.standard_normal(n ** 3)
+    p = cb.make_params(3, n, n * dx, 4.0, 0.1 * dx, precision="fp64", memorysave=1)
+    monkeypatch.setenv("CB_TEMPORAL_BLOCK", "2")
+    two = cb.Bubble(p, *start)
+    monkeypatch.setenv("CB_TEMPORAL_BLOCK", "1")
+    one = cb.Bubble(p, *start)
+    for k in (2, 7):
+        a, b = two.step(k, sums=k != 2), one.step(k, sums=k != 2)
+        assert a == b
+        fa, fb = two.fields(), one.fields()
+        np.testing.assert_array_equal(fa["phi"], fb["phi"])
+        np.testing.assert_array_equal(fa["pi"], fb["pi"])
+    assert two.counters() == (1 + 4, 9) and one.counters() == (9, 9)
