@@ -101,10 +101,10 @@ extern "C" int cb_step_static_noalloc(const cb_params *p, const void *phi_in, co
     cudaError_t e = cudaMemcpyAsync(st, &s, sizeof s, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) {
         const int prec = p->precision == CB_FP64 ? P_FP64 : P_FP32;
-        /* the kernel a run's reporting step takes; its vector copies want 16-byte
-         * buffers, the caller's need not be */
-        const bool vectors = (((uintptr_t)phi_in | (uintptr_t)pi_in | (uintptr_t)phi_out | (uintptr_t)pi_out) & 15) == 0;
-        if (vectors && step2tb_steps(k, prec, 1, true) == 1)
+        /* the kernel a run's reporting step takes; those of vectors and bulk copies want
+         * 16-byte buffers, which the caller's need not be: the generic one takes any */
+        if ((((uintptr_t)phi_in | (uintptr_t)pi_in | (uintptr_t)phi_out | (uintptr_t)pi_out) & 15) != 0) k.force_generic = 1;
+        if (step2tb_steps(k, prec, 1, true) == 1)
             e = launch_step2_tb(prec, k, 1, true, phi_in, pi_in, phi_out, pi_out, st, partials, stream);
         else
             e = launch_step(prec, k, false, SUM_FULL, phi_in, pi_in, phi_out, pi_out, nullptr, nullptr, nullptr, st,
