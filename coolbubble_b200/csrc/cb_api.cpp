@@ -362,17 +362,25 @@ void destroy_handle(cb_handle *h) {
     delete h;
 }
 
-/* Elements of the staging buffer that padded fields go through (a lattice's
- * worth would not fit beside the largest ones). */
+/* Rows at a time that padded fields go through the staging buffer in: some 2^26
+ * elements (a lattice's worth would not fit beside the largest ones), fewer where
+ * the device has no room for them. */
 constexpr size_t STAGED_ELEMS = size_t(1) << 26;
+int stage_rows(cb_handle *h, size_t elem_bytes, size_t &most) {
+    const size_t n = (size_t)h->p.n_grids;
+    most = std::max<size_t>(1, std::min(h->N / n, STAGED_ELEMS / n));
+    int r;
+    while ((r = ensure_tmp(h, most * n * elem_bytes)) != CB_OK && most > 1) most = (most + 1) / 2;
+    return r;
+}
 
 /* Download a field of padded rows into dense host memory of the given type;
  * waits for each piece. */
 cudaError_t download_padded(cb_handle *h, const void *src, int to_prec, void *dst, int &status) {
     const size_t n = (size_t)h->p.n_grids, pitch = (size_t)h->k.pitch, rows = h->N / n;
     const size_t osz = to_prec == P_FP64 ? sizeof(double) : sizeof(float);
-    const size_t most = std::max<size_t>(1, std::min(rows, STAGED_ELEMS / n));
-    if ((status = ensure_tmp(h, most * n * osz)) != CB_OK) return cudaSuccess;
+    size_t most;
+    if ((status = stage_rows(h, osz, most)) != CB_OK) return cudaSuccess;
     cudaError_t e = cudaSuccess;
     for (size_t at = 0; at < rows && e == cudaSuccess; at += most) {
         const size_t m = std::min(most, rows - at);
@@ -393,8 +401,8 @@ int upload_field(cb_handle *h, void *dst, const double *src) {
     const size_t n = (size_t)h->p.n_grids, pitch = (size_t)h->k.pitch, rows = h->N / n;
     if (pitch != n) {
         /* padded rows: dense pieces through a bounded staging buffer */
-        const size_t most = std::max<size_t>(1, std::min(rows, STAGED_ELEMS / n));
-        int r = ensure_tmp(h, most * n * sizeof(double));
+        size_t most;
+        int r = stage_rows(h, sizeof(double), most);
         if (r != CB_OK) return r;
         for (size_t at = 0; at < rows && e == cudaSuccess; at += most) {
             const size_t m = std::min(most, rows - at);

@@ -28,6 +28,7 @@ int fail_at = -1;         /* ... and this one of them fails */
 
 int waits = 0, ones = 0, twos = 0;   /* waits for a stream or event, one-step and two-step launches */
 bool two_step = false;               /* the two-step pass applies */
+size_t room = (size_t)-1;            /* bytes of an allocation that still fit */
 
 void run_stream(cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
@@ -56,7 +57,9 @@ extern "C" void *aligned_alloc(size_t align, size_t bytes) {
 }
 
 extern "C" {
-cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
+cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) {
+    return n <= room && (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation;
+}
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return std::free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaFreeHost(void *p) { return std::free(p), cudaSuccess; }
@@ -115,7 +118,13 @@ cudaError_t launch_flush_drift(int, const StepConst &, const void *, const void 
 cudaError_t launch_ic_backkick(int, const StepConst &, const void *, void *, DevState *, double *, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_ic_energies(int, const StepConst &, const void *, const void *, void *, void *, void *, DevState *, double *,
                                cudaStream_t) { return cudaSuccess; }
-cudaError_t launch_repitch(int, int, const void *, size_t, void *, size_t, int, size_t, cudaStream_t) { return cudaSuccess; }
+/* between rows of doubles */
+cudaError_t launch_repitch(int from, int to, const void *src, size_t sp, void *dst, size_t dp, int n, size_t rows, cudaStream_t s) {
+    run_stream(s);
+    for (size_t r = 0; from == P_FP64 && to == P_FP64 && r < rows; ++r)
+        std::memcpy((double *)dst + r * dp, (const double *)src + r * sp, n * sizeof(double));
+    return cudaSuccess;
+}
 cudaError_t launch_step(int, const StepConst &, bool, int, const void *, const void *, void *, void *, void *, void *, void *,
                         DevState *, double *, cudaStream_t) { return ++ones, cudaSuccess; }
 cudaError_t launch_step2_tb(int, const StepConst &, int, bool, const void *, const void *, void *, void *, DevState *, double *,
@@ -214,6 +223,22 @@ int first_steps(int n, int precision) {
     return cb_destroy(h) == CB_OK ? 0 : 1;
 }
 
+/* Padded rows on a device with little room beside the fields: they go up and come
+ * down in smaller pieces. */
+int little_room(int n) {
+    const cb_params p = params(3, n, CB_FP64);
+    const size_t sites = (size_t)n * n * n, field = (size_t)n * n * (n + 1) * sizeof(double);
+    std::vector<double> start(sites), phi(sites), pi(sites);
+    for (size_t i = 0; i < sites; ++i) start[i] = 0.25 + (double)i;
+    cb_handle *h = nullptr;
+    CHECK(cb_create_from_ic(&p, start.data(), start.data(), nullptr, &h) == CB_OK);
+    room = field / 7;   /* the staging buffer was released after the set-up */
+    CHECK(cb_get_fields(h, phi.data(), pi.data(), nullptr, nullptr, nullptr) == CB_OK);
+    CHECK(phi == start && pi == start);
+    room = (size_t)-1;
+    return cb_destroy(h) == CB_OK ? 0 : 1;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -222,6 +247,7 @@ int main(int argc, char **argv) {
     if (what == "download") bad = download(2, 64, CB_FP32C) || download(2, 64, CB_FP64) || download(3, 65, CB_FP32C);
     else if (what == "served") bad = served(1500, 0) || served(1500, 1) || served(64, 1);
     else if (what == "first") bad = first_steps(64, CB_FP64) || first_steps(65, CB_FP32C) || first_steps(128, CB_FP32C);
+    else if (what == "room") bad = little_room(65);
     else bad = std::printf("what?\n");
     std::printf(bad ? "failed\n" : "ok\n");
     return bad ? 1 : 0;

@@ -1,5 +1,5 @@
 """The library's host code on a fake of the CUDA runtime (no GPU): downloads that
-fail half-way, and what a run's first steps launch."""
+fail half-way or find little room, and what a run's first steps launch."""
 import os
 import subprocess
 
@@ -34,3 +34,7 @@ def test_a_served_run_without_its_fields_hands_out_zeros(fake):
 
 def test_first_steps_launch_their_steps_and_wait_for_nothing(fake):
     run(fake, "first")
+
+
+def test_padded_fields_come_down_where_the_device_has_little_room(fake):
+    run(fake, "room")
