@@ -202,10 +202,6 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * elsewhere they are too few and keeping it costs more than reading it back (250^3 float 27.7 -> 26.3 us per step,
      * 192^3 15.6 -> 14.7; 512^3, NV, 170 -> 174) */
     constexpr bool KEEP_Y = NV != 0;
-    /* 64 bits for the registers the compiler then assigns: 256^3 double 56.2 -> 55.3 us
-     * per step, while the general rows are faster with 32 (250^3 float 28.3 -> 27.7,
-     * double 61.2 -> 60.4) */
-    using Count = std::conditional_t<NV != 0 && std::is_same<T, double>::value, long long, int>;
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ int abort_flag;
     __shared__ int item_q[TB_IQ];
@@ -245,7 +241,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * its start up to the lattice's last row, then the rest from row 0 */
     __shared__ size_t pr_r[2];   /* thread 0's only: kept out of the registers */
     __shared__ int pr_c[2];
-    Count issued = 0;                                            /* planes issued so far */
+    int issued = 0;                                              /* planes issued so far */
     int is_stage = 0;                                            /* its stage: issued mod nstage */
     bool pr_done = false;
     auto next_item = [&]() {
@@ -270,7 +266,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         pr_c[0] = min(R0, n - r0);
         pr_c[1] = min(R0p, n - r1);
     };
-    auto issue_upto = [&](Count last) {
+    auto issue_upto = [&](int last) {
         while (!pr_done && issued <= last) {
             const int s = is_stage;
             const int pw = pr_pl < 0 ? pr_pl + n : (pr_pl >= n ? pr_pl - n : pr_pl);
@@ -357,20 +353,23 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
      * runs in any case (what it stores belongs to a step reported as failed); in
      * double, where the registers come out better for it, whole warps skip it.
      * us per step with the skip and without, float: 192^3 14.9 and 14.2, 250^3 26.4
-     * and 25.5, 512^3 172 and 172; double: 192^3 28.7 and 27.2, 250^3 61.1 and 63.4,
-     * 256^3 56.4 and 56.6. */
+     * and 25.5, 512^3 172 and 172; double: 192^3 28.4 and 27.2, 250^3 60.9 and 63.4,
+     * 320^3 127 and 130. */
     constexpr bool SKIP = std::is_same<T, double>::value;
     bool bad = false;
     auto acquire = [&]() -> bool {
         const bool ok = mbar_wait(&full[gs], gph, WAIT_LIMIT);
-        if (!ok) atomicExch(&abort_flag, 1);
-        bad = !ok;
+        if (!ok) {
+            atomicExch(&abort_flag, 1);
+            if (SKIP) bad = true;
+        }
+        if (!SKIP) bad = !ok;
         return !SKIP || warp_all(ok);
     };
     /* end of round g: every thread's reads of the planes and level-1 slots are
      * done and its level-1 writes visible; thread 0 then issues the planes
      * whose stages that freed. Returns whether any thread's wait ran out. */
-    auto end_round = [&](Count g, bool bad) -> bool {
+    auto end_round = [&](int g, bool bad) -> bool {
         const bool any_bad = tb_any(bad);
         if (!any_bad && threadIdx.x == 0) issue_upto(g + nstage - 1);
         return any_bad;
@@ -378,7 +377,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
     Slot<V> sl[TB_NTS];
     HT hxm, hxc;
     auto at = [&](int s) { return off0 + s * slot_step; };
-    Count g = 0;   /* the round: index of the input plane it waits for */
+    int g = 0;   /* the round: index of the input plane it waits for */
     for (int j = 0;; ++j) {
         const int it = item_q[j % TB_IQ];
         if (it < 0) break;
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(TB_MAXT, 1)
         /* record, then let every issued copy land before the block exits */
         if (threadIdx.x == 0) {
             atomicExch(&st->err, ERR_TMA_TIMEOUT);
-            for (int q = max((int)issued - nstage, 0); q < (int)issued; ++q)
+            for (int q = max(issued - nstage, 0); q < issued; ++q)
                 mbar_wait(&full[q % nstage], (uint32_t)((q / nstage) & 1), WAIT_LIMIT / 8);
         }
         __syncthreads();
