@@ -28,9 +28,9 @@
  * What bounds it: the arithmetic of the tile, halo included. ncu, 8 steps on
  * 4096^2 floats: FMA pipe 62 % busy (the packed operations occupy it two
  * cycles), DRAM 21 %; 4 steps on 3072^2 doubles: FP64 pipe 60-65 %, DRAM 32 %.
- * us per step, one launch per step -> here: 512^2 double 2.72 -> 1.07, 1000^2
- * float 6.69 -> 1.25, 3072^2 double (dx^2 no power of two) 52.2 -> 24.5,
- * 4096^2 float 47.3 -> 13.4; 4096 sites (d = 1, double) 2.19 -> 0.16.
+ * us per step, one launch per step -> here: 512^2 double 2.72 -> 1.05, 1000^2
+ * float 6.69 -> 1.23, 3072^2 double (dx^2 no power of two) 52.2 -> 24.6,
+ * 4096^2 float 47.3 -> 13.4; 4096 sites (d = 1, double) 2.19 -> 0.14.
  *
  * The per-site operations are those of the one-step kernels (cb_step.cu,
  * cb_step2.cu) for a = 1, where a^(d-2) = a^d = 1 and the products with them
