@@ -31,10 +31,6 @@
 
 using namespace cb;
 
-namespace cb {
-void fill_sums(const cb_handle *h, const DevState &s, cb_sums *o);
-}
-
 struct cb_ensemble {
     std::vector<cb_handle *> members;
     /* members of one precision and kind, stepped by the same launches */
@@ -310,14 +306,14 @@ int cb_ensemble_step(cb_ensemble *e, int nsteps, int sums_every, cb_sums *out) {
                 h->launches += b.launches;
             }
         for (int i = 0; i < count; ++i) {
-            const cb_handle *h = e->members[i];
+            cb_handle *h = e->members[i];
             double t = t_start[i];
             for (int j = 0; j < nev; ++j) {
                 for (int q = 0; q < sums_every; ++q) t += h->p.dt;
                 cb_sums &o = out[(size_t)i * nev + j];
                 std::memset(&o, 0, sizeof o);
-                fill_sums(h, rec[(size_t)i * nev + j], &o);
-                o.t = t;
+                const int r = sums_from_record(h, rec[(size_t)i * nev + j], t, &o);
+                if (r != CB_OK) return fail(nullptr, r, "cb_ensemble_step: " + h->err);
             }
         }
         return CB_OK;

@@ -1,4 +1,4 @@
-/* A CUDA runtime on the host for cb_api.cpp and cb_pool.cpp: "device" memory is
+/* A CUDA runtime on the host for cb_api.cpp, cb_pool.cpp and cb_ensemble.cu: "device" memory is
  * host memory, kernels do nothing, and copies to the host stay queued on their
  * stream until it is waited for. A test can make one of those copies fail. Built
  * and run by test_host_path.py, which needs no GPU. */
@@ -29,6 +29,7 @@ int fail_at = -1;         /* ... and this one of them fails */
 int waits = 0, ones = 0, twos = 0;   /* waits for a stream or event, one-step and two-step launches */
 bool two_step = false;               /* the two-step pass applies */
 size_t room = (size_t)-1;            /* bytes of an allocation that still fit */
+int timed_out = 0;                   /* error word that a step leaves in the record */
 
 void run_stream(cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
@@ -60,6 +61,10 @@ extern "C" {
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) {
     return n <= room && (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation;
 }
+cudaError_t cudaMalloc(void **p, size_t n) { return cudaMallocAsync(p, n, nullptr); }
+cudaError_t cudaFree(void *p) { return std::free(p), cudaSuccess; }
+cudaError_t cudaMemcpy(void *dst, const void *src, size_t n, cudaMemcpyKind) { return std::memcpy(dst, src, n), cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return std::free(p), cudaSuccess; }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { return (*p = std::calloc(1, n)) ? cudaSuccess : cudaErrorMemoryAllocation; }
 cudaError_t cudaFreeHost(void *p) { return std::free(p), cudaSuccess; }
@@ -113,6 +118,14 @@ size_t step_blocks(const StepConst &) { return 1; }
 int step2tb_steps(const StepConst &, int, int, bool) { return 0; }
 bool step3df_applies(const StepConst &, int) { return false; }
 bool step3tb_geometry(const StepConst &, int, int tl, int &, int &, size_t &, unsigned &, int &) { return two_step && tl == 2; }
+/* no member of these tests is batched */
+int batch2_kind(const StepConst &, int) { return 0; }
+int batch2_steps(const std::vector<int> &, int, int, int) { return 0; }
+int batch2_threads(const std::vector<int> &, int, int, int) { return 0; }
+std::vector<int> batch2_tiles(const std::vector<int> &, int, int, int) { return {}; }
+cudaError_t launch_step2_batch(int, int, const Batch2Member *, const std::vector<int> &, int, int, int, double *, cudaStream_t) {
+    return cudaErrorNotSupported;
+}
 cudaError_t launch_convert(int, int, const void *, void *, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_flush_drift(int, const StepConst &, const void *, const void *, void *, DevState *, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_ic_backkick(int, const StepConst &, const void *, void *, DevState *, double *, cudaStream_t) { return cudaSuccess; }
@@ -126,7 +139,10 @@ cudaError_t launch_repitch(int from, int to, const void *src, size_t sp, void *d
     return cudaSuccess;
 }
 cudaError_t launch_step(int, const StepConst &, bool, int, const void *, const void *, void *, void *, void *, void *, void *,
-                        DevState *, double *, cudaStream_t) { return ++ones, cudaSuccess; }
+                        DevState *st, double *, cudaStream_t) {
+    if (timed_out) st->err = timed_out;
+    return ++ones, cudaSuccess;
+}
 cudaError_t launch_step2_tb(int, const StepConst &, int, bool, const void *, const void *, void *, void *, DevState *, double *,
                             cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_step3_df(int, const StepConst &, int, bool, void *, void *, void *, void *, DevState *, double *,
@@ -239,6 +255,23 @@ int little_room(int n) {
     return cb_destroy(h) == CB_OK ? 0 : 1;
 }
 
+/* An ensemble whose member's step ended in a wait that ran out says so. */
+int ensemble_timeout() {
+    const cb_params p = params(3, 16, CB_FP64);
+    std::vector<double> start(16 * 16 * 16, 0.5);
+    cb_handle *h = nullptr;
+    cb_ensemble *e = nullptr;
+    cb_sums lines[4];
+    CHECK(cb_create_from_ic(&p, start.data(), nullptr, nullptr, &h) == CB_OK);
+    CHECK(cb_ensemble_create(1, &h, &e) == CB_OK);
+    CHECK(cb_ensemble_step(e, 4, 2, lines) == CB_OK);
+    timed_out = 0x71;
+    CHECK(cb_ensemble_step(e, 4, 2, lines) == CB_ETIMEOUT);
+    timed_out = 0;
+    CHECK(cb_ensemble_destroy(e) == CB_OK);
+    return cb_destroy(h) == CB_OK ? 0 : 1;
+}
+
 }  // namespace
 
 int main(int argc, char **argv) {
@@ -247,6 +280,7 @@ int main(int argc, char **argv) {
     if (what == "download") bad = download(2, 64, CB_FP32C) || download(2, 64, CB_FP64) || download(3, 65, CB_FP32C);
     else if (what == "served") bad = served(1500, 0) || served(1500, 1) || served(64, 1);
     else if (what == "first") bad = first_steps(64, CB_FP64) || first_steps(65, CB_FP32C) || first_steps(128, CB_FP32C);
+    else if (what == "ensemble") bad = ensemble_timeout();
     else if (what == "room") bad = little_room(65);
     else bad = std::printf("what?\n");
     std::printf(bad ? "failed\n" : "ok\n");

@@ -15,7 +15,8 @@ def fake(tmp_path_factory):
     cuda = os.environ.get("CUDA", "/usr/local/cuda")
     subprocess.run(["g++", "-std=c++17", "-O1", "-I" + CSRC, "-I" + os.path.join(ROOT, "include"),
                     "-I" + os.path.join(cuda, "include"), os.path.join(ROOT, "tests", "native", "fake_cuda.cpp"),
-                    os.path.join(CSRC, "cb_api.cpp"), os.path.join(CSRC, "cb_pool.cpp"), "-o", exe, "-lpthread"], check=True)
+                    os.path.join(CSRC, "cb_api.cpp"), os.path.join(CSRC, "cb_pool.cpp"), "-x", "c++",
+                    os.path.join(CSRC, "cb_ensemble.cu"), "-o", exe, "-lpthread"], check=True)
     return exe
 
 
@@ -38,3 +39,7 @@ def test_first_steps_launch_their_steps_and_wait_for_nothing(fake):
 
 def test_padded_fields_come_down_where_the_device_has_little_room(fake):
     run(fake, "room")
+
+
+def test_an_ensemble_reports_a_member_whose_wait_ran_out(fake):
+    run(fake, "ensemble")
