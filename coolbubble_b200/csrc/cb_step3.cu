@@ -189,9 +189,9 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
     constexpr bool FULL = SUMS == SUM_FULL || SUMS == SUM_LINE;
     constexpr int NS = FULL ? NSUM : 3;                /* sums carried (S_EK, S_EP, S_EG first) */
     /* float with padded rows: every site's term in double, as the generic kernel, which took
-     * them before, compensates each (a reporting step of 250^3 89 us; 69 with a vector's
+     * them before, compensates each (a reporting step of 250^3 70 us; 69 with a vector's
      * terms added in float first, 180 in the generic kernel; plain expanding steps of 250^3
-     * 52.6 and 52.3 with the Friedmann sums' pairs added in float) */
+     * 52.6 and 52.2 with the Friedmann sums' pairs added in float) */
     constexpr bool DSUM = RAG && SUMS != SUM_NONE && std::is_same<T, float>::value;
     extern __shared__ __align__(128) unsigned char smraw[];
     const int n = NV ? NV * W : k.n, np = RAG ? k.pitch : n;   /* sites and elements of a row */
@@ -603,19 +603,30 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                                     v23[q] = f2_pack(sites > 2 ? f2_lo(v23[q]) : 0.f, 0.f);
                                 }
                             }
+                            if constexpr (DSUM) {
+                                /* each term converted once: for its sum and, squared there, for its spread
+                                 * (converted again for the spread, a line of 250^3 took 20 us more) */
+                                auto put = [&](int sum, int square, F2 x, F2 y) {
+                                    const float f[4] = {f2_lo(x), f2_hi(x), f2_lo(y), f2_hi(y)};
+    #pragma unroll
+                                    for (int i = 0; i < 4; ++i) {
+                                        const double d = (double)f[i];
+                                        if (sum >= 0) dacc[sum] = __dadd_rn(dacc[sum], d);
+                                        if (square >= 0) dacc[square] = __fma_rn(d, d, dacc[square]);
+                                    }
+                                };
+                                put(S_EK, FULL ? Q_EK : -1, v01[S_EK], v23[S_EK]);
+                                put(S_EP, FULL ? Q_EP : -1, v01[S_EP], v23[S_EP]);
+                                if constexpr (want_eg) put(S_EG, FULL ? Q_EG : -1, v01[S_EG], v23[S_EG]);
+                                if constexpr (FULL) {
+                                    put(-1, Q_ET, v01[Q_ET], v23[Q_ET]);
+                                    put(S_PHI, Q_PHI, v01[S_PHI], v23[S_PHI]);
+                                    put(S_V, Q_V, v01[S_V], v23[S_V]);
+                                    put(S_EKIN_IN, -1, v01[S_EKIN_IN], v23[S_EKIN_IN]);
+                                }
+                            } else {
     #pragma unroll
                             for (int q = 0; q < NA; ++q) {
-                                if constexpr (DSUM) {
-                                    F2 x = v01[q], y = v23[q];
-                                    if (q >= Q_EK && q <= Q_V) {
-                                        x = f2_mul(x, x);
-                                        y = f2_mul(y, y);
-                                    }
-                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_lo(x));
-                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_hi(x));
-                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_lo(y));
-                                    dacc[q] = __dadd_rn(dacc[q], (double)f2_hi(y));
-                                } else
                                 /* the energies (and the previous half step's kinetic sum, which
                                  * enters the time-centred Ekin) are compensated, per half of the
                                  * pair; the field averages and the sums of squares behind the
@@ -628,6 +639,7 @@ __global__ void __launch_bounds__(NT3, 2) k_step3(StepConst k, int tj_, int nsta
                                     pacc[q] = f2_fma(v23[q], v23[q], f2_fma(v01[q], v01[q], pacc[q]));
                                 else
                                     pacc[q] = f2_add(pacc[q], f2_add(v01[q], v23[q]));
+                            }
                             }
                             if constexpr (SUMS == SUM_FULL) {
                                 vek = make_float4(f2_lo(v01[S_EK]), f2_hi(v01[S_EK]), f2_lo(v23[S_EK]), f2_hi(v23[S_EK]));
